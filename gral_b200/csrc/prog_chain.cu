@@ -1,0 +1,982 @@
+// prog_chain.cu -- row-chain schedule of the slab family's Gauss-Seidel sweeps.
+//
+// A sweep is two launches.  A parallel kernel evaluates every column's coefficients and sources
+// (all that does not read values the sweep itself changes), runs the forward elimination and writes
+// one contiguous record per column.  The chain kernel then walks the sweep rows i1, a row's columns
+// j1 in order, and passes finished columns on as stamped words (float bits and a stamp in one 8-byte
+// access): through rings in shared memory inside a block and to the next block of the cluster,
+// through global memory from one cluster's claim to the next.
+//
+// What bounds it: the chain of (rows + columns) column steps.  A step's time is two first-order
+// vertical recurrences over about 40 levels, whose every operation is rounded as in the reference.
+// Run one level after the other they take about 20 (back-substitution) and 12 (Q) cycles a level.
+// Here a lane holds levels 2*lane and 2*lane+1 and the warp iterates x_k = f_k(x_k-1) on all
+// levels at once, each round passing values two levels on through one shuffle, until a whole round
+// changes no bit.  A state that f maps to itself, starting from the exact first level, is the
+// sequential recurrence's result bit for bit (by induction over the levels), whatever the number of
+// rounds; the recurrences are contractions (the influence of a level fades by relax*P <= 0.1 or
+// by C*T, well below 1), so a few rounds reach it instead of forty levels.
+//
+// A claim (the strips of one cluster) is taken from an atomic counter in order and waits only on the
+// claim before, so clusters need not be resident together; the blocks of a cluster are.  Every wait
+// is bounded and gives up when another warp has set the error word.
+#include <algorithm>
+#include <cmath>
+
+#include "prog_common.cuh"
+#include "prog_kernels.cuh"
+#include "prog_level.cuh"
+
+namespace gral {
+
+namespace {
+
+constexpr int CH_RING = 8;    // hand-off slots between a row and the row below it in the block
+constexpr int CH_AHEAD = 4;   // columns of a warp whose records are asked into L2 ahead
+constexpr int CT_COLS = 32;   // columns of a tile of the coefficient kernels
+constexpr int CT_THREADS = 256;
+
+enum { COMP_U = 0, COMP_V = 1, COMP_W = 2 };
+
+// A column record of the momentum sweeps: pairs of values per level, [pair][KMAX_LEVELS] float2, so
+// that a lane reads its two levels of a pair with one 16-byte load at a constant offset (levels from
+// KS up are never touched).  The sweep's direction is known when
+// the record is written, so it names the neighbours by what the chain knows of them: cI, cJ are the
+// coefficients of the predecessors (i-IS, j) and (i, j-JS), kI and kJ what the successors contribute.
+template <int COMP, int SW>
+__host__ __device__ constexpr int mom_pairs() { return COMP == COMP_W ? 7 : ((COMP == COMP_V && SW == 8) ? 9 : 10); }
+constexpr int MOM_PAIRS_MAX = 10;
+// level flags of a record (bits of a float)
+enum : unsigned { L_Q = 1u, L_U = 2u, L_X = 4u, L_VEG = 8u };
+
+__device__ __forceinline__ void chain_dir(int it, int &IS, int &JS) {
+    // PrognosticFlowfield.cs:770-802
+    const int m = it % 4;
+    IS = (m == 0 || m == 1) ? -1 : 1;
+    JS = (m == 1 || m == 2) ? -1 : 1;
+}
+
+// What a chain step needs of one level: the sums of DIM in the reference's order, split into the
+// parts the predecessors enter (see MomChain::dim).
+struct LevelRec {
+    float cI, cJ, kI, kJ, t1, t2, t3, w, vdx, K, e0, e1, e2, e3, phi, C, T, P, sI;
+    unsigned fl;
+};
+// pair q of a record as the two values stored at a level
+template <int COMP, int SW>
+__device__ __forceinline__ float2 rec_pair(const LevelRec &r, int q) {
+    const float fl = __uint_as_float(r.fl);
+    if (COMP == COMP_W) {
+        switch (q) {
+            case 0: return make_float2(r.cI, r.cJ);
+            case 1: return make_float2(r.kI, r.kJ);
+            case 2: return make_float2(r.t1, r.t2);
+            case 3: return make_float2(r.t3, r.e0);
+            case 4: return make_float2(r.phi, fl);
+            case 5: return make_float2(r.C, r.sI);
+            default: return make_float2(r.T, r.P);
+        }
+    }
+    switch (q) {
+        case 0: return make_float2(r.cI, r.cJ);
+        case 1: return make_float2(r.kI, r.kJ);
+        case 2: return make_float2(r.t1, r.t2);
+        case 3: return make_float2(r.t3, r.w);
+        case 4: return make_float2(r.vdx, r.K);
+        case 5: return make_float2(r.e0, r.e1);
+        case 6: return make_float2(r.e2, r.C);
+        case 7: return make_float2(r.phi, fl);
+        case 8: return make_float2(r.T, r.P);
+        default: return make_float2(r.e3, r.sI);
+    }
+}
+template <int COMP, int SW>
+__device__ __forceinline__ void rec_unpair(LevelRec &r, int q, float2 v) {
+    if (COMP == COMP_W) {
+        switch (q) {
+            case 0: r.cI = v.x; r.cJ = v.y; break;
+            case 1: r.kI = v.x; r.kJ = v.y; break;
+            case 2: r.t1 = v.x; r.t2 = v.y; break;
+            case 3: r.t3 = v.x; r.e0 = v.y; break;
+            case 4: r.phi = v.x; r.fl = __float_as_uint(v.y); break;
+            case 5: r.C = v.x; r.sI = v.y; break;
+            default: r.T = v.x; r.P = v.y; break;
+        }
+        return;
+    }
+    switch (q) {
+        case 0: r.cI = v.x; r.cJ = v.y; break;
+        case 1: r.kI = v.x; r.kJ = v.y; break;
+        case 2: r.t1 = v.x; r.t2 = v.y; break;
+        case 3: r.t3 = v.x; r.w = v.y; break;
+        case 4: r.vdx = v.x; r.K = v.y; break;
+        case 5: r.e0 = v.x; r.e1 = v.y; break;
+        case 6: r.e2 = v.x; r.C = v.y; break;
+        case 7: r.phi = v.x; r.fl = __float_as_uint(v.y); break;
+        case 8: r.T = v.x; r.P = v.y; break;
+        default: r.e3 = v.x; r.sI = v.y; break;
+    }
+}
+template <int COMP>
+__host__ __device__ constexpr int tp_pair() { return COMP == COMP_W ? 6 : 8; }   // the pair that holds T and P
+
+// ------------------------------------ coefficients ------------------------------------------
+
+// Tile of a coefficient launch: CT_COLS columns along j of one sweep row of one unit.
+struct Tile {
+    int u, s, i, j0, nc, IS, JS;
+    bool ok;
+};
+__device__ __forceinline__ Tile make_tile(const KArgs &a, const SweepGeom &g, const ChainBufs &b, bool reverse) {
+    Tile t;
+    chain_dir(*a.it_global, t.IS, t.JS);
+    if (reverse) { t.IS = -t.IS; t.JS = -t.JS; }
+    const int per = (g.nj + CT_COLS - 1) / CT_COLS;
+    const int q = blockIdx.x / per;
+    const int c0 = (blockIdx.x - q * per) * CT_COLS;
+    t.u = q / g.ni;
+    const int i1 = g.ia + (q - t.u * g.ni);
+    t.i = (t.IS == 1) ? i1 : a.nii - i1 + 1;
+    t.nc = min(CT_COLS, g.nj - c0);
+    // the tile's columns in ascending j: sweep columns j1 = ja + c0 ... of either direction
+    t.j0 = (t.JS == 1) ? g.ja + c0 : a.njj - (g.ja + c0 + t.nc - 1) + 1;
+    t.ok = b.unit_lo + t.u < *a.nact;
+    t.s = t.ok ? a.act[b.unit_lo + t.u] : 0;
+    t.ok = t.ok && a.sit[t.s].active;
+    return t;
+}
+
+// The record of one level from its coefficients: products and sums that involve only the successors'
+// old values are formed here, each where the reference's association order allows it.
+template <int COMP, int SW>
+__device__ __forceinline__ void level_rec(LevelRec &r, const MomPre &p, int IS, int JS, float sI, float sJ, bool veg,
+                                          bool extra) {
+    const float cs = IS == 1 ? p.ae : p.aw;          // coefficient of the successor in i
+    r.cI = IS == 1 ? p.aw : p.ae;
+    r.cJ = JS == 1 ? p.as : p.an;
+    r.kI = cs * sI;
+    r.kJ = (JS == 1 ? p.an : p.as) * sJ;
+    if (SW == 16 && (COMP != COMP_V || veg)) {       // pairs by fused multiply-add (the Vector512 twins)
+        if (IS == JS) r.kI = fmaf(cs, sI, r.kJ);     // the pair of both successors
+        else r.kI = cs;                              // the successor in i pairs with the predecessor in j
+    } else if (IS == -1 && JS == -1) {
+        r.kI = r.kI + r.kJ;                          // AW1*PHI + AS1*PHI, the first two of the sum
+    }
+    r.sI = sI;
+    r.t1 = p.t1; r.t2 = p.t2; r.t3 = p.t3;
+    if (COMP == COMP_U && SW == 16 && !veg) {        // + fma(DDPX, DYKDZK, t3); adding -0 changes nothing
+        r.t2 = fmaf(p.t2, p.hz, p.t3);
+        r.t3 = -0.0f;
+    }
+    r.phi = p.phi; r.C = p.C;
+    r.e0 = extra ? p.e0 : 0.0f;
+    if (COMP != COMP_W) {
+        r.w = p.w; r.vdx = p.vdx;
+        r.e1 = extra ? p.e1 : 0.0f;
+        r.e2 = extra ? p.e2 : 0.0f;
+        if (COMP == COMP_U) {
+            r.e3 = extra ? p.e3 : 0.0f;
+            r.K = IS == 1 ? (sI - p.phi) * p.hz : (p.phi - sI) * p.hz;      // DUDXE or DUDXW
+        } else {
+            r.K = JS == 1 ? r.e0 + (sJ - p.phi) * p.hz : (p.phi - sJ) * p.hz;   // e0 + DVDYN, or DVDYS
+        }
+    }
+}
+
+// Coefficients of one model-1 momentum sweep.  Threads map to (column, level) pairs in the slab's
+// memory order, so loads and record stores are contiguous and no lane idles below KS levels; the
+// forward elimination P_k = B_k*T_k, T_k = 1/(A_k - C_k*P_k-1) then runs with a lane per column
+// (32 independent serial chains per warp) on rows in shared memory.
+template <int COMP, int SW>
+__global__ void __launch_bounds__(CT_THREADS, 3) k_mom1_terms(KArgs a, SweepGeom g, ChainBufs b) {
+    __shared__ float sA[CT_COLS][KMAX_LEVELS + 1], sB[CT_COLS][KMAX_LEVELS + 1], sC[CT_COLS][KMAX_LEVELS + 1];
+    const Tile t = make_tile(a, g, b, COMP == COMP_V);
+    if (!t.ok) return;
+    constexpr int NP = mom_pairs<COMP, SW>(), TP = tp_pair<COMP>();
+    constexpr int KL = KMAX_LEVELS;
+    const int ks = a.ks;
+    const SitCtx sc = make_sit(a, t.s);
+    const float *F = COMP == COMP_U ? a.uk : (COMP == COMP_V ? a.vk : a.wk);
+    constexpr size_t rs = (size_t)NP * KL;     // float2 of a record
+    float2 *base = b.rec + ((size_t)t.u * a.ncols + (size_t)(t.i * a.nj2 + t.j0)) * rs;
+    for (int q = threadIdx.x; q < t.nc * ks; q += CT_THREADS) {
+        const int cl = q / ks, k = q - cl * ks;
+        const ColCtx c = make_col(a, t.i, t.j0 + cl);
+        const Acc<false> x = make_acc<false>(a, t.s, c.col);
+        float2 *rec = base + (size_t)cl * rs + k;
+        LevelRec r;
+        if (!(c.fl & F_ADV) || k < c.K0 || k > c.VI) {     // a level the sweep does not change
+            r.phi = F[x.at(0, k)];
+            r.fl = 0u;
+            constexpr int PP = COMP == COMP_W ? 4 : 7;
+            rec[PP * KL] = rec_pair<COMP, SW>(r, PP);
+            continue;
+        }
+        MomPre p;
+        if (COMP == COMP_U) p = u1_pre<false, SW>(a, x, c, sc, k);
+        else if (COMP == COMP_V) p = v1_pre<false, SW>(a, x, c, sc, k);
+        else p = w1_pre<false, SW>(a, x, c, sc, k);
+        sA[cl][k] = p.A; sB[cl][k] = p.B; sC[cl][k] = p.C;
+        const float sI = F[x.at((long long)t.IS * c.nj2, k)], sJ = F[x.at((long long)t.JS, k)];
+        const bool veg = (c.fl & F_VEG) != 0, extra = k >= c.kad;
+        level_rec<COMP, SW>(r, p, t.IS, t.JS, sI, sJ, veg, extra);
+        const int kkm = COMP == COMP_U ? c.kkm_u : (COMP == COMP_V ? c.kkm_v : -1);
+        r.fl = (k > c.KK + 1 ? L_Q : 0u) | (k > kkm ? L_U : 0u) | (extra ? L_X : 0u) | (veg ? L_VEG : 0u);
+#pragma unroll
+        for (int n = 0; n < NP; ++n)
+            if (n != TP) rec[n * KL] = rec_pair<COMP, SW>(r, n);
+    }
+    __syncthreads();
+    if (threadIdx.x < t.nc) {
+        const int cl = threadIdx.x, col = t.i * a.nj2 + t.j0 + cl;
+        const ColMeta m = a.meta[col];
+        if (a.cflags[col] & F_ADV) {
+            float P = 0.0f;
+            for (int k = m.kstart; k <= m.vi; ++k) {
+                const float A = sA[cl][k], B = sB[cl][k], C = sC[cl][k];
+                const float T = (k > m.kkart + 1) ? 1.0f / (A - C * P) : 1.0f / A;
+                P = B * T;
+                sA[cl][k] = T;
+                sB[cl][k] = P;
+            }
+        }
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < t.nc * ks; q += CT_THREADS) {
+        const int cl = q / ks, k = q - cl * ks;
+        base[(size_t)cl * rs + TP * KL + k] = make_float2(sA[cl][k], sB[cl][k]);
+    }
+}
+
+// Divergence term DIV/DTIME of the pressure sweep, [unit][col][KS].
+__global__ void __launch_bounds__(CT_THREADS) k_pressure_terms(KArgs a, SweepGeom g, ChainBufs b) {
+    const Tile t = make_tile(a, g, b, false);
+    if (!t.ok) return;
+    const int ks = a.ks;
+    const SitCtx sc = make_sit(a, t.s);
+    float *base = reinterpret_cast<float *>(b.rec) + ((size_t)t.u * a.ncols + (size_t)(t.i * a.nj2 + t.j0)) * ks;
+    for (int q = threadIdx.x; q < t.nc * ks; q += CT_THREADS) {
+        const int cl = q / ks, k = q - cl * ks;
+        ColCtx c;
+        c.nj2 = a.nj2; c.i = t.i; c.j = t.j0 + cl;
+        c.col = c.i * a.nj2 + c.j;
+        const ColMeta m = a.meta[c.col];
+        c.KK = m.kkart; c.VI = m.vi;
+        if (!(a.cflags[c.col] & F_ADV) || k <= c.KK || k > c.VI) continue;
+        base[q] = pressure_pre<false>(a, make_acc<false>(a, t.s, c.col), c, sc, k);
+    }
+}
+
+// Forward elimination of the pressure sweep, T = 1/(APP - ATP*P) and P = ABP*T from VerticalIndex
+// down to KKART+1, per i-direction: [dir][col][KS] {T, P}, zero on the levels the sweep does not
+// change.  It depends on the grid alone, so it is built once per load.  A column starts from the P
+// that its row-carry writer (rcw) left at VerticalIndex+1, zero without one.  Every thread takes a
+// column and passes are repeated until one changes nothing; the start's influence fades by P*P a
+// level, so two or three passes suffice.  A pass after the first only recomputes the top level and
+// stops there if it is unchanged.
+__global__ void __launch_bounds__(128) k_pressure_tab(KArgs a, float2 *tab, int *changed, int pass) {
+    if (pass > 0 && changed[pass - 1] == 0) return;
+    const int dir = blockIdx.y, ks = a.ks;
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= a.ncols) return;
+    const int i = col / a.nj2, j = col - i * a.nj2;
+    if (i < 2 || i > a.nii - 1 || j < 2 || j > a.njj - 1 || !(a.cflags[col] & F_ADV)) return;
+    const ColMeta m = a.meta[col];
+    float2 *tp = tab + ((size_t)dir * a.ncols + col) * ks;
+    const short2 w = a.rcw[col];
+    const int wi = dir == 0 ? w.x : w.y;
+    float P = 0.0f;
+    if (wi >= 0) P = *(volatile float *)&tab[((size_t)dir * a.ncols + (size_t)wi * a.nj2 + j) * ks + m.vi + 1].y;
+    for (int k = m.vi; k > m.kkart; --k) {
+        const float T = 1.0f / (a.app[k] - a.atp[k] * P);
+        P = a.abp[k] * T;
+        if (pass > 0 && __float_as_uint(T) == __float_as_uint(tp[k].x)) return;   // the rest follows from T
+        tp[k] = make_float2(T, P);
+        if (k == m.vi) changed[pass] = 1;
+    }
+}
+
+// ------------------------------------ row chains --------------------------------------------
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// Stamped words of two neighbouring levels.
+struct Words2 {
+    unsigned long long a, b;
+};
+__device__ __forceinline__ unsigned long long word(float v, unsigned stamp) {
+    return ((unsigned long long)stamp << 32) | __float_as_uint(v);
+}
+__device__ __forceinline__ float word_val(unsigned long long w) { return __uint_as_float((unsigned)w); }
+__device__ __forceinline__ bool stamped(const Words2 &w, unsigned stamp) {
+    return (unsigned)(w.a >> 32) == stamp && (unsigned)(w.b >> 32) == stamp;
+}
+// The accesses of a lane without levels (`on` false) are predicated off rather than branched over:
+// a branch costs the chain a reconvergence.
+__device__ __forceinline__ Words2 ld_words(const unsigned long long *p, bool on) {
+    Words2 w;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.u64 %0, 0;\n\tmov.u64 %1, 0;\n\t"
+        "@q ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];\n\t}"
+        : "=&l"(w.a), "=&l"(w.b)
+        : "l"(p), "r"((unsigned)on)
+        : "memory");
+    return w;
+}
+__device__ __forceinline__ void st_words(unsigned long long *p, const Words2 &w, bool on) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};\n\t}" ::"l"(p),
+        "l"(w.a), "l"(w.b), "r"((unsigned)on)
+        : "memory");
+}
+__device__ __forceinline__ void st_pair(float2 *p, float2 v, bool on) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q st.global.cg.v2.f32 [%0], {%1, %2};\n\t}" ::"l"(p),
+                 "f"(v.x), "f"(v.y), "r"((unsigned)on)
+                 : "memory");
+}
+__device__ __forceinline__ Words2 lds_words(unsigned p) {
+    Words2 w;
+    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(w.a), "=l"(w.b) : "r"(p) : "memory");
+    return w;
+}
+__device__ __forceinline__ void sts_words(unsigned p, const Words2 &w) {
+    asm volatile("st.volatile.shared.v2.u64 [%0], {%1, %2};" ::"r"(p), "l"(w.a), "l"(w.b) : "memory");
+}
+__device__ __forceinline__ void l2_ahead(const void *p, bool on) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q prefetch.global.L2 [%0];\n\t}" ::"l"(p),
+                 "r"((unsigned)on));
+}
+// d = a + b or a * b where `on`, as one predicated instruction: the compiler's own forms of a
+// conditional assignment (a select after the operation, or a branch over it) lengthen the recurrences
+// (a round of the momentum step took 109 cycles with `if`, 80 with a select, 68 this way).
+__device__ __forceinline__ void add_if(float &d, float a, float b, unsigned on) {
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q add.rn.f32 %0, %1, %2;\n\t}" : "+f"(d) : "f"(a), "f"(b), "r"(on));
+}
+__device__ __forceinline__ void mul_if(float &d, float a, float b, unsigned on) {
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q mul.rn.f32 %0, %1, %2;\n\t}" : "+f"(d) : "f"(a), "f"(b), "r"(on));
+}
+__device__ __forceinline__ bool differ(float a, float b) { return __float_as_uint(a) != __float_as_uint(b); }
+
+// Bound of a spin: every 32nd call looks at the error word and the clock; true when the wait must
+// end (warp-uniform).
+struct SpinBound {
+    unsigned long long t0 = 0;
+    unsigned n = 0;
+    __device__ __forceinline__ bool expired(const KArgs &a) {
+        if (n == 0) t0 = globaltimer_ns();
+        if ((++n & 31) != 0) return false;
+        bool stop = *(volatile int *)a.err != ERR_NONE;
+        if (!stop && globaltimer_ns() - t0 > a.wait_limit_ns) {
+            atomicCAS(a.err, ERR_NONE, ERR_TIMEOUT);
+            stop = true;
+        }
+        return __any_sync(0xffffffffu, stop);
+    }
+};
+
+// Rounds of the two recurrences before the first test; a failed test continues round by round.  One
+// round less or more: 400x400 U chain 0.45 / 0.42 / 0.45 ms for 4 / 3 / 2, pressure 0.58 / 0.57 / 0.60 for
+// 5 / 6 / 4 (the pressure's influence fades by 0.17 a level where the layers are as thick as wide).
+constexpr int ROUNDS_MOM = 3, ROUNDS_PRESS = 6;
+
+// Model-1 momentum: record of one column in registers (two levels per lane) and the step, for one
+// sweep direction (branches on it would stall the chain).
+template <int COMP, int SW, int IS, int JS>
+struct MomChain {
+    static constexpr int NV = 1;                    // values handed to the row below
+    static constexpr int NP = mom_pairs<COMP, SW>();
+    struct Rec {
+        float4 f[NP];      // {x(2l), y(2l), x(2l+1), y(2l+1)} of each pair
+    };
+    struct Val {
+        float2 v[NV];
+    };
+    float relax;
+    float2 hz;
+    float *F;
+    const float4 *rec;     // this lane's part of the next record to load
+    const char *line;      // this lane's 128-byte line of the next record to ask into L2
+    bool on0, on1;         // whether the line exists (and the one 32 lines on)
+
+    __device__ __forceinline__ void init(const KArgs &a, int lane) {
+        relax = a.relax;
+        F = COMP == COMP_U ? a.uk : (COMP == COMP_V ? a.vk : a.wk);
+        const float face = COMP == COMP_U ? a.dyk : a.dxk;
+        const int l = min(lane, a.ks / 2 - 1);
+        hz = make_float2(face * a.dzk[2 * l], face * a.dzk[2 * l + 1]);
+        on0 = (lane & 3) * 16 < a.ks && (lane >> 2) < NP;
+        on1 = (lane & 3) * 16 < a.ks && (lane >> 2) + 8 < NP;
+    }
+    int step_rec;          // float4 to this warp's next record
+    template <int M>
+    __device__ __forceinline__ void begin(const KArgs &a, const ChainBufs &b, int u, int col, int lane) {
+        step_rec = JS * M * (NP * (KMAX_LEVELS / 2));
+        const float2 *p = b.rec + ((size_t)u * a.ncols + col) * (NP * KMAX_LEVELS);
+        rec = reinterpret_cast<const float4 *>(p) + min(lane, a.ks / 2 - 1);
+        line = reinterpret_cast<const char *>(p) + 128 * lane;
+    }
+    // asks the next column's record into L2; loads the next column's record
+    __device__ __forceinline__ void ahead(bool on) {
+        l2_ahead(line, on && on0);
+        if (NP > 8) l2_ahead(line + 4096, on && on1);
+        line += step_rec * 16;
+    }
+    __device__ __forceinline__ void load(Rec &r) {
+#pragma unroll
+        for (int q = 0; q < NP; ++q) r.f[q] = __ldcg(rec + q * (KMAX_LEVELS / 2));
+        rec += step_rec;
+    }
+    // the field's values of a column that this sweep does not change
+    __device__ __forceinline__ Val still(const KArgs &a, size_t base, int lane) const {
+        Val o;
+        o.v[0] = __ldcg(reinterpret_cast<const float2 *>(F + base) + min(lane, a.ks / 2 - 1));
+        return o;
+    }
+    // DIM of one level: the neighbour products and sources in the reference's association order
+    __device__ __forceinline__ float dim(const LevelRec &r, float hzk, float vI, float vJ) const {
+        float D;
+        const float pJ = r.cJ * vJ;
+        float Df = 0.0f;
+        if (SW == 16) {   // U-prognostic-microscale_1_Vec512.cs:399-421
+            float S1, S2;
+            if (IS == JS) {
+                S1 = fmaf(r.cI, vI, pJ);
+                S2 = r.kI;                                    // a + b == b + a: either pair may come first
+            } else {
+                S1 = fmaf(r.cI, vI, r.kJ);
+                S2 = fmaf(r.kI, r.sI, pJ);
+            }
+            Df = S1 + S2;
+        }
+        if (SW == 8 || COMP == COMP_V) {
+            const float pI = r.cI * vI;
+            if (IS == 1) D = (JS == 1) ? pI + pJ + r.kI + r.kJ : pI + r.kJ + r.kI + pJ;
+            else D = (JS == 1) ? r.kI + pJ + pI + r.kJ : r.kI + pI + pJ;
+            if (SW == 16 && (r.fl & L_VEG)) D = Df;
+        } else {
+            D = Df;
+        }
+        D = D + r.t1 + r.t2;
+        if (COMP == COMP_W) {
+            D = D - r.t3;
+            add_if(D, D, r.e0, r.fl & L_X);
+            return D;
+        }
+        D = D + r.t3 - r.w;
+        float X;
+        if (COMP == COMP_U) {
+            const float d = (IS == 1) ? r.K - (r.phi - vI) * hzk : (vI - r.phi) * hzk - r.K;
+            X = d + r.e0 - r.e1 + r.e2 - r.e3;
+        } else {
+            const float d = (JS == 1) ? r.K - (r.phi - vJ) * hzk : r.e0 + (vJ - r.phi) * hzk - r.K;
+            X = d + r.e1 - r.e2;
+        }
+        add_if(D, D, r.vdx * X, r.fl & L_X);
+        return D;
+    }
+    __device__ __forceinline__ Val step(const Rec &rc, const Val &vI, const float2 &vJ) const {
+        LevelRec A, B;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            rec_unpair<COMP, SW>(A, q, make_float2(rc.f[q].x, rc.f[q].y));
+            rec_unpair<COMP, SW>(B, q, make_float2(rc.f[q].z, rc.f[q].w));
+        }
+        const float Da = dim(A, hz.x, vI.v[0].x, vJ.x), Db = dim(B, hz.y, vI.v[0].y, vJ.y);
+        // Q_k = D_k*T_k up to KKART+1, above it Q_k = (D_k + C_k*Q_k-1)*T_k
+        const unsigned qA = A.fl & L_Q, qB = B.fl & L_Q, uA = A.fl & L_U, uB = B.fl & L_U;
+        float Qa = Da * A.T, Qb = Db * B.T, inQ = 0.0f, inU = 0.0f;
+        mul_if(Qb, Db + B.C * Qa, B.T, qB);
+        auto up = [&]() {
+            mul_if(Qa, Da + A.C * inQ, A.T, qA);
+            mul_if(Qb, Db + B.C * Qa, B.T, qB);
+        };
+        // relaxed back-substitution from VerticalIndex down; the other levels keep their value
+        float va = A.phi, vb = B.phi;
+        auto down = [&]() {
+            add_if(vb, B.phi, relax * (B.P * inU + Qb - B.phi), uB);
+            add_if(va, A.phi, relax * (A.P * vb + Qa - A.phi), uA);
+        };
+        // while Q settles, the back-substitution already iterates on the Q of the round before: its
+        // chain runs beside Q's, and little is left for it once Q is final
+#pragma unroll
+        for (int n = 0; n < ROUNDS_MOM; ++n) {
+            inU = __shfl_down_sync(0xffffffffu, va, 1);
+            inQ = __shfl_up_sync(0xffffffffu, Qb, 1);
+            down();
+            up();
+        }
+        for (;;) {
+            const float nU = __shfl_down_sync(0xffffffffu, va, 1), nQ = __shfl_up_sync(0xffffffffu, Qb, 1);
+            const bool more = __any_sync(0xffffffffu, differ(nQ, inQ));
+            inU = nU; inQ = nQ;
+            down();
+            if (!more) break;      // Q is final, and this round used it
+            up();
+        }
+        for (;;) {
+            const float nU = __shfl_down_sync(0xffffffffu, va, 1);
+            const bool more = __any_sync(0xffffffffu, differ(nU, inU));
+            inU = nU;
+            down();
+            if (!more) break;
+        }
+        Val o;
+        o.v[0] = make_float2(va, vb);
+        return o;
+    }
+};
+
+// Pressure correction (PrognosticFlowfield.cs:804-901).  Values handed on: DPM and the row carry's Q
+// (the reference's QIMP buffer lives per sweep row j and is not cleared between columns, :865-868:
+// a column's Q starts from what an earlier column of its row j left at VerticalIndex+1), which
+// therefore travels along i with the DPM.  DPMNEW and the residual follow in the velocity correction.
+template <int IS, int JS, bool P2>
+struct PressChain {
+    static constexpr int NV = 2;
+    struct Rec {
+        float4 tp;      // {T, P} of the two levels
+        float2 d;       // DIV/DTIME
+    };
+    struct Val {
+        float2 v[NV];
+    };
+    float2 atp, dz;
+    float dxk, dyk, rx, ry;
+    float *F;
+    const float2 *div;
+    const float4 *tab;
+    const char *line;
+    long long step_line;
+    int hstep;
+    bool on0;
+
+    __device__ __forceinline__ void init(const KArgs &a, int lane) {
+        F = a.dpm;
+        dxk = a.dxk; dyk = a.dyk;
+        rx = 1.0f / dxk; ry = 1.0f / dyk;
+        const int l = min(lane, a.ks / 2 - 1);
+        atp = make_float2(a.atp[2 * l], a.atp[2 * l + 1]);
+        dz = make_float2(a.dzk[2 * l], a.dzk[2 * l + 1]);
+    }
+    template <int M>
+    __device__ __forceinline__ void begin(const KArgs &a, const ChainBufs &b, int u, int col, int lane) {
+        hstep = JS * M * (a.ks / 2);
+        const int l = min(lane, a.ks / 2 - 1);
+        const float *d = reinterpret_cast<const float *>(b.rec) + ((size_t)u * a.ncols + col) * a.ks;
+        const float2 *t = b.ptab + ((size_t)(IS == 1 ? 0 : 1) * a.ncols + col) * a.ks;
+        div = reinterpret_cast<const float2 *>(d) + l;
+        tab = reinterpret_cast<const float4 *>(t) + l;
+        // lines of 128 bytes of the two runs (they need not start on one): lanes 0-3 and 4-9
+        line = lane < 4 ? reinterpret_cast<const char *>(d) + 128 * lane : reinterpret_cast<const char *>(t) + 128 * (lane - 4);
+        on0 = lane < 4 ? 128 * lane < a.ks * 4 : (lane < 8 && 128 * (lane - 4) < a.ks * 8);
+        step_line = (long long)JS * M * a.ks * (lane < 4 ? 4 : 8);
+    }
+    __device__ __forceinline__ void ahead(bool on) {
+        l2_ahead(line, on && on0);
+        line += step_line;
+    }
+    __device__ __forceinline__ void load(Rec &r) {
+        r.tp = __ldcg(tab);
+        r.d = __ldcg(div);
+        tab += hstep;
+        div += hstep;
+    }
+    // outside the sweep DPM is zero, and a sweep row's carry starts from zero
+    __device__ __forceinline__ Val still(const KArgs &, size_t, int) const {
+        Val o;
+        o.v[0] = o.v[1] = make_float2(0.0f, 0.0f);
+        return o;
+    }
+    // pressure_post_v of one level
+    __device__ __forceinline__ float dim(float t0, float dzk, float pi, float pj) const {
+        const float si = (IS == 1) ? (pi + 0.0f) : (0.0f + pi);
+        const float sj = (JS == 1) ? (pj - 0.0f) : (0.0f - pj);
+        // x / 2^n == x * 2^-n in every rounding, so power-of-two spacings (P2) need no division
+        const float qi = P2 ? si * rx : si / dxk, qj = P2 ? sj * ry : sj / dyk;
+        return t0 + qi * dyk * dzk + qj * dxk * dzk;
+    }
+    __device__ __forceinline__ Val step(const Rec &r, const Val &vI, const float2 &vJ) const {
+        const float Ta = r.tp.x, Pa = r.tp.y, Tb = r.tp.z, Pb = r.tp.w;
+        const unsigned lA = Ta != 0.0f, lB = Tb != 0.0f;
+        const float Da = dim(r.d.x, dz.x, vI.v[0].x, vJ.x), Db = dim(r.d.y, dz.y, vI.v[0].y, vJ.y);
+        // Q downwards from the carry at VerticalIndex+1
+        float Qa = vI.v[1].x, Qb = vI.v[1].y, inQ = 0.0f, inD = 0.0f;
+        mul_if(Qb, Db, Tb, lB);
+        mul_if(Qa, atp.x * Qb + Da, Ta, lA);
+        auto down = [&]() {
+            mul_if(Qb, atp.y * inQ + Db, Tb, lB);
+            mul_if(Qa, atp.x * Qb + Da, Ta, lA);
+        };
+        // DPM upwards from the zero at KKART
+        float da = 0.0f, db = 0.0f;
+        auto up = [&]() {
+            add_if(da, Pa * inD, Qa, lA);
+            add_if(db, Pb * da, Qb, lB);
+        };
+        // the two recurrences side by side, as in the momentum step
+#pragma unroll
+        for (int n = 0; n < ROUNDS_PRESS; ++n) {
+            inD = __shfl_up_sync(0xffffffffu, db, 1);
+            inQ = __shfl_down_sync(0xffffffffu, Qa, 1);
+            up();
+            down();
+        }
+        for (;;) {
+            const float nD = __shfl_up_sync(0xffffffffu, db, 1), nQ = __shfl_down_sync(0xffffffffu, Qa, 1);
+            const bool more = __any_sync(0xffffffffu, differ(nQ, inQ));
+            inD = nD; inQ = nQ;
+            up();
+            if (!more) break;      // Q is final, and this round used it
+            down();
+        }
+        for (;;) {
+            const float nD = __shfl_up_sync(0xffffffffu, db, 1);
+            const bool more = __any_sync(0xffffffffu, differ(nD, inD));
+            inD = nD;
+            up();
+            if (!more) break;
+        }
+        Val o;
+        o.v[0] = make_float2(da, db);
+        o.v[1] = make_float2(Qa, Qb);
+        return o;
+    }
+};
+
+// Bytes of a ring slot (every lane's words of one column) and of a ring in shared memory.
+template <int NV>
+__host__ __device__ constexpr unsigned slot_bytes() { return NV * 32u * 16u; }
+template <int NV>
+__host__ __device__ constexpr unsigned ring_bytes() { return CH_RING * slot_bytes<NV>(); }
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// address of this block's shared-memory location p in block `rank` of the cluster
+__device__ __forceinline__ unsigned remote(unsigned p, unsigned rank) {
+    unsigned q;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(q) : "r"(p), "r"(rank));
+    return q;
+}
+__device__ __forceinline__ void st_remote(unsigned p, const Words2 &w, bool on) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};\n\t}" ::"r"(p),
+        "l"(w.a), "l"(w.b), "r"((unsigned)on)
+        : "memory");
+}
+__device__ __forceinline__ void st_remote(unsigned p, int v, bool on) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.relaxed.cluster.shared::cluster.s32 [%0], %1;\n\t}" ::"r"(p),
+                 "r"(v), "r"((unsigned)on)
+                 : "memory");
+}
+__device__ __forceinline__ unsigned ld_remote(unsigned p) {
+    unsigned v;
+    asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+    return v;
+}
+
+// Shared memory of a block: the rings 0..SR (ring r: what row r takes from above; ring SR: what the
+// strip's last row finished), the claim, and how many columns each ring's reader has taken.
+template <int SR, int NV>
+struct ChainSmem {
+    alignas(16) unsigned long long ring[(SR + 1) * ring_bytes<NV>() / 8];
+    unsigned claim;
+    int taken[SR + 1];
+};
+
+// One cluster of CL blocks takes CL strips of SR rows each (a claim), M warps per row: warp m of a
+// row runs the columns m, m+M, ..., so that while one warp is in its step the row's other warps
+// store, ask for their next record and load it.  A finished column goes into the ring of the row
+// below, where that row and the next column's warp of this row read it; from the last row of a
+// strip also into ring 0 of the next block of the cluster, and from the last row of the claim into
+// the words in global memory, which the feeder warp of the next claim's first block turns into its
+// ring 0 (for the sweep's first row: the values the sweep does not change).
+template <class Job, int PH, int SR, int M, int CL, int IS, int JS>
+__device__ __forceinline__ void run_chain(const KArgs &a, const SweepGeom &g, const ChainBufs &b,
+                                          ChainSmem<SR, Job::NV> &sm) {
+    constexpr int NV = Job::NV;
+    constexpr int WCOL = NV * KMAX_LEVELS;        // words of a column in global memory
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ks = a.ks, nj = g.nj, l2 = 2 * lane;
+    const bool mine = l2 < ks;       // this lane holds levels of the column
+    const unsigned rank = cluster_rank();
+    const unsigned ring0 = smem_u32(sm.ring) + lane * 16u;
+    Job job;
+    job.init(a, lane);
+    const unsigned gstamp = (unsigned)*b.epoch * 8u + PH;      // of the words in global memory
+    const unsigned units = (unsigned)min(b.unit_n, max(0, *a.nact - b.unit_lo));
+    const unsigned ngroups = (unsigned)((g.ni + SR * CL - 1) / (SR * CL));
+    const unsigned total = ngroups * units;
+    unsigned *ctr = a.counters + 8 * b.ctr_slot + PH;
+    unsigned seq = 0;                // claims run by this block: part of the ring stamps
+    const int jfirst = (JS == 1) ? g.ja : a.njj - g.ja + 1;
+    const size_t wrow = (size_t)nj * WCOL;
+    for (;;) {
+        cluster_sync();
+        if (rank == 0 && threadIdx.x == 0)
+            sm.claim = (*(volatile int *)a.err != ERR_NONE) ? 0xffffffffu : atomicAdd(ctr, 1u);
+        if (threadIdx.x <= SR) sm.taken[threadIdx.x] = 0;
+        cluster_sync();
+        const unsigned t = ld_remote(remote(smem_u32(&sm.claim), 0));
+        if (t >= total) break;
+        ++seq;
+        const int u = (int)(t % units), group = (int)(t / units);
+        const int s = a.act[b.unit_lo + u];
+        const int first = g.ia + (group * CL + (int)rank) * SR, rows = min(SR, g.ia + g.ni - first);
+        if (!a.sit[s].active || rows <= 0) continue;
+        auto row_i = [&](int r) { return (IS == 1) ? first + r : a.nii - (first + r) + 1; };
+        unsigned long long *gout = b.words + ((size_t)(b.unit_lo + u) * ngroups + group) * wrow + l2;
+        const unsigned sbase = seq << 16;
+        // waits until ring r's reader has taken n columns (their slots are free)
+        int seen = 0;
+        auto room = [&](int r, int n) {
+            if (seen >= n) return true;
+            SpinBound sb;
+            for (;;) {
+                seen = __shfl_sync(0xffffffffu, *(volatile int *)(sm.taken + r), 0);
+                if (seen >= n) return true;
+                if (sb.expired(a)) return false;
+            }
+        };
+        auto slot = [&](int c) { return (unsigned)(c & (CH_RING - 1)) * slot_bytes<NV>(); };
+        auto push = [&](unsigned ring, int c, const typename Job::Val &v) {
+            const unsigned st = sbase + (unsigned)(c + 1), p = ring + slot(c);
+#pragma unroll
+            for (int q = 0; q < NV; ++q) sts_words(p + q * 512u, Words2{word(v.v[q].x, st), word(v.v[q].y, st)});
+        };
+        if (warp == SR * M) {                                      // the feeder
+            constexpr int NF = 4;                                  // columns in flight
+            bool ok = true;
+            if (rank > 0) {
+            } else if (group > 0) {
+                const unsigned long long *gin = gout - wrow;
+                Words2 w[NF][NV];
+                auto peek = [&](int c, Words2 (&x)[NV]) {
+#pragma unroll
+                    for (int q = 0; q < NV; ++q) x[q] = ld_words(gin + (size_t)c * WCOL + q * KMAX_LEVELS, mine && c < nj);
+                };
+                auto feed = [&](int c, Words2 (&x)[NV]) {
+                    SpinBound sb;
+                    for (;;) {
+                        bool got = true;
+#pragma unroll
+                        for (int q = 0; q < NV; ++q) got = got && stamped(x[q], gstamp);
+                        if (__all_sync(0xffffffffu, got || !mine)) break;
+                        if (sb.expired(a)) return false;
+                        peek(c, x);
+                    }
+                    typename Job::Val v;
+#pragma unroll
+                    for (int q = 0; q < NV; ++q) v.v[q] = make_float2(word_val(x[q].a), word_val(x[q].b));
+                    if (!room(0, c - CH_RING + 1)) return false;
+                    push(ring0, c, v);
+                    peek(c + NF, x);
+                    return true;
+                };
+#pragma unroll
+                for (int q = 0; q < NF; ++q) peek(q, w[q]);
+                for (int c = 0; c < nj && ok; c += NF)
+#pragma unroll
+                    for (int q = 0; q < NF; ++q)
+                        if (ok && c + q < nj) ok = feed(c + q, w[q]);
+            } else {
+                const int cb = (row_i(0) - IS) * a.nj2 + jfirst;
+                auto value = [&](int c) {
+                    return job.still(a, ((size_t)s * a.ncols + (size_t)(cb + JS * min(c, nj - 1))) * ks, lane);
+                };
+                typename Job::Val v[NF];
+#pragma unroll
+                for (int q = 0; q < NF; ++q) v[q] = value(q);
+                for (int c = 0; c < nj && ok; c += NF)
+#pragma unroll
+                    for (int q = 0; q < NF; ++q)
+                        if (ok && c + q < nj) {
+                            ok = room(0, c + q - CH_RING + 1);
+                            push(ring0, c + q, v[q]);
+                            v[q] = value(c + q + NF);
+                        }
+            }
+            continue;
+        }
+        const int r = warp / M, m = warp - r * M;
+        if (r >= rows) continue;
+        const bool more_rows = first + rows < g.ia + g.ni;             // a strip follows this one
+        const bool last = r + 1 == rows;                               // the strip's last row
+        const bool next_block = last && more_rows && rank + 1 < CL;    // ... read by the cluster's next block
+        const bool next_claim = last && more_rows && rank + 1 == CL && mine;
+        const unsigned ring_in = ring0 + (unsigned)r * ring_bytes<NV>(), ring_out = ring_in + ring_bytes<NV>();
+        const unsigned ring_far = remote(ring0, min(rank + 1, CL - 1u));
+        const unsigned taken_far = remote(smem_u32(sm.taken + SR), max((int)rank, 1) - 1);
+        const bool far_above = r == 0 && rank > 0 && lane == 0;        // this row reads the block before
+        const bool watch = !last || next_block;                        // somebody reads this row's columns
+        const int taker = last ? SR : r + 1;
+        const int col0 = row_i(r) * a.nj2 + jfirst;
+        const size_t e0 = ((size_t)s * a.ncols + (size_t)col0) * ks;
+        float2 *out_f = reinterpret_cast<float2 *>(job.F + e0) + lane + (long long)m * JS * (ks / 2);
+        unsigned long long *wout = gout + (size_t)m * WCOL;
+        job.template begin<M>(a, b, u, col0 + JS * m, lane);
+        if (m == 0) push(ring_out, -1, job.still(a, e0 - (long long)JS * ks, lane));   // left of the first column
+        typename Job::Rec rec;
+        for (int c = m; c < m + CH_AHEAD * M; c += M) job.ahead(c < nj);
+        if (m < nj) job.load(rec);
+        for (int c = m; c < nj; c += M) {
+            Words2 wI[NV], wJ;
+            const unsigned want = sbase + (unsigned)(c + 1), pI = ring_in + slot(c), pJ = ring_out + slot(c - 1);
+            SpinBound sb;
+            bool ok = true;
+            for (;;) {
+                wJ = lds_words(pJ);
+#pragma unroll
+                for (int q = 0; q < NV; ++q) wI[q] = lds_words(pI + q * 512u);
+                bool got = stamped(wJ, want - 1u);
+#pragma unroll
+                for (int q = 0; q < NV; ++q) got = got && stamped(wI[q], want);
+                if (__all_sync(0xffffffffu, got)) break;
+                if (sb.expired(a)) { ok = false; break; }
+            }
+            typename Job::Val vI;
+#pragma unroll
+            for (int q = 0; q < NV; ++q) vI.v[q] = make_float2(word_val(wI[q].a), word_val(wI[q].b));
+            const typename Job::Val v = job.step(rec, vI, make_float2(word_val(wJ.a), word_val(wJ.b)));
+            if (!ok) break;
+            push(ring_out, c, v);
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                const unsigned st = sbase + (unsigned)(c + 1);
+                st_remote(ring_far + slot(c) + q * 512u, Words2{word(v.v[q].x, st), word(v.v[q].y, st)}, next_block);
+            }
+            // the rest runs while the row's next column is in its step
+            *(volatile int *)(sm.taken + r) = c + 1;
+            st_remote(taken_far, c + 1, far_above);
+            if (c + M < nj) job.load(rec);
+#pragma unroll
+            for (int q = 0; q < NV; ++q)
+                st_words(wout + q * KMAX_LEVELS, Words2{word(v.v[q].x, gstamp), word(v.v[q].y, gstamp)}, next_claim);
+            st_pair(out_f, v.v[0], mine);     // levels the sweep does not change keep their value
+            wout += (size_t)M * WCOL;
+            out_f += M * JS * (ks / 2);
+            job.ahead(c + CH_AHEAD * M < nj);
+            if (watch && !room(taker, c + M - CH_RING + 1)) break;
+        }
+    }
+    cluster_sync();      // no block leaves while another may still write into its shared memory
+}
+
+// Strip shape: rows of a block, warps of a row, blocks of a cluster.  Measured on the 400x400 grid,
+// ms of an iteration: (4,2,8) 3.44, (3,2,8) 3.51, (2,3,8) 3.61, (4,3,8) 3.48; one warp per row and every
+// hand-off between blocks through global memory 4.25.
+constexpr int CH_SR = 4, CH_M = 2, CH_CL = 8;
+constexpr int CH_THREADS = (CH_SR * CH_M + 1) * 32;
+
+// The kernels take the sweep's direction from the iteration count and run the code built for it.
+template <int COMP, int SW>
+__global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 1) k_mom_chain(KArgs a, SweepGeom g, ChainBufs b) {
+    __shared__ ChainSmem<CH_SR, 1> sm;
+    constexpr int PH = COMP == COMP_U ? PH_U : (COMP == COMP_V ? PH_V : PH_W);
+    constexpr int SR = CH_SR, M = CH_M, CL = CH_CL;
+    for (unsigned q = threadIdx.x; q < sizeof(sm.ring) / 8; q += CH_THREADS) sm.ring[q] = 0ull;
+    int is, js;
+    chain_dir(*a.it_global, is, js);
+    if (COMP == COMP_V) { is = -is; js = -js; }     // model-1 V sweeps with (-IS,-JS)
+    if (is == 1) {
+        if (js == 1) run_chain<MomChain<COMP, SW, 1, 1>, PH, SR, M, CL, 1, 1>(a, g, b, sm);
+        else run_chain<MomChain<COMP, SW, 1, -1>, PH, SR, M, CL, 1, -1>(a, g, b, sm);
+    } else {
+        if (js == 1) run_chain<MomChain<COMP, SW, -1, 1>, PH, SR, M, CL, -1, 1>(a, g, b, sm);
+        else run_chain<MomChain<COMP, SW, -1, -1>, PH, SR, M, CL, -1, -1>(a, g, b, sm);
+    }
+}
+
+template <bool P2>
+__global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 1) k_pressure_chain(KArgs a, SweepGeom g, ChainBufs b) {
+    __shared__ ChainSmem<CH_SR, 2> sm;
+    constexpr int PH = PH_PRESSURE, SR = CH_SR, M = CH_M, CL = CH_CL;
+    for (unsigned q = threadIdx.x; q < sizeof(sm.ring) / 8; q += CH_THREADS) sm.ring[q] = 0ull;
+    int is, js;
+    chain_dir(*a.it_global, is, js);
+    if (is == 1) {
+        if (js == 1) run_chain<PressChain<1, 1, P2>, PH, SR, M, CL, 1, 1>(a, g, b, sm);
+        else run_chain<PressChain<1, -1, P2>, PH, SR, M, CL, 1, -1>(a, g, b, sm);
+    } else {
+        if (js == 1) run_chain<PressChain<-1, 1, P2>, PH, SR, M, CL, -1, 1>(a, g, b, sm);
+        else run_chain<PressChain<-1, -1, P2>, PH, SR, M, CL, -1, -1>(a, g, b, sm);
+    }
+}
+
+using KFn = void (*)(KArgs, SweepGeom, ChainBufs);
+
+bool pow2(float x) {
+    int e;
+    return std::frexp(x, &e) == 0.5f && e > -100 && e < 100;
+}
+
+KFn chain_kernel(int kind, const KArgs &a) {
+    const bool w = a.simd == 16;
+    switch (kind) {
+        case PH_PRESSURE: return (pow2(a.dxk) && pow2(a.dyk)) ? k_pressure_chain<true> : k_pressure_chain<false>;
+        case PH_U: return w ? k_mom_chain<COMP_U, 16> : k_mom_chain<COMP_U, 8>;
+        case PH_V: return w ? k_mom_chain<COMP_V, 16> : k_mom_chain<COMP_V, 8>;
+        default: return w ? k_mom_chain<COMP_W, 16> : k_mom_chain<COMP_W, 8>;
+    }
+}
+
+KFn terms_kernel(int kind, int simd) {
+    const bool w = simd == 16;
+    switch (kind) {
+        case PH_PRESSURE: return k_pressure_terms;
+        case PH_U: return w ? k_mom1_terms<COMP_U, 16> : k_mom1_terms<COMP_U, 8>;
+        case PH_V: return w ? k_mom1_terms<COMP_V, 16> : k_mom1_terms<COMP_V, 8>;
+        default: return w ? k_mom1_terms<COMP_W, 16> : k_mom1_terms<COMP_W, 8>;
+    }
+}
+
+}  // namespace
+
+size_t chain_record_bytes() { return (size_t)MOM_PAIRS_MAX * KMAX_LEVELS * sizeof(float2); }
+
+size_t chain_unit_words(int nii, int njj) {
+    return (size_t)chain_claims(nii - 2) * (njj - 2) * 2 * KMAX_LEVELS;   // two values a level at most
+}
+
+int chain_claims(int ni) { return (ni + CH_SR * CH_CL - 1) / (CH_SR * CH_CL); }
+
+cudaError_t chain_grid(int kind, const KArgs &a, long long claims, int *grid) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CH_CL);
+    cfg.blockDim = dim3(CH_THREADS);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CH_CL;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, chain_kernel(kind, a), &cfg);
+    if (e != cudaSuccess) return e;
+    *grid = CH_CL * (int)std::max<long long>(1, std::min<long long>(std::max(1, clusters), claims));
+    return cudaSuccess;
+}
+
+void launch_chain(int kind, const KArgs &a, const SweepGeom &g, const ChainBufs &bufs, int grid, cudaStream_t st) {
+    if (g.ni <= 0 || g.nj <= 0) return;
+    ChainBufs b = bufs;
+    b.ctr_slot = 0;
+    for (b.unit_lo = 0; b.unit_lo < a.nb; b.unit_lo += bufs.unit_n, ++b.ctr_slot) {
+        const int n = std::min(bufs.unit_n, a.nb - b.unit_lo);
+        const long long tiles = (long long)n * g.ni * ((g.nj + CT_COLS - 1) / CT_COLS);
+        terms_kernel(kind, a.simd)<<<(unsigned)tiles, CT_THREADS, 0, st>>>(a, g, b);
+        chain_kernel(kind, a)<<<grid, CH_THREADS, 0, st>>>(a, g, b);
+    }
+}
+
+void launch_pressure_tab(const KArgs &a, float2 *tab, int *changed, int first, int passes, cudaStream_t st) {
+    for (int p = first; p < first + passes; ++p)
+        k_pressure_tab<<<dim3((a.ncols + 127) / 128, 2), 128, 0, st>>>(a, tab, changed, p);
+}
+
+}  // namespace gral

@@ -117,6 +117,8 @@ struct KArgs {
     const int *act;                      // active situation list (slab layout)
     const int *nact;                     // number of active situations
     int *it_global;                      // IterationLoops of the batch (all situations in lockstep)
+    int *epoch;                          // iterations run in this context (row-chain schedule), or null
+    int chain;                           // row-chain schedule: the velocity correction updates DPMNEW and the residual
     unsigned long long wait_limit_ns;    // bound of every spin wait
     int chunk;                           // tasks claimed per atomic
     float *trace;                        // [nb][trace_cap] DeltaUMax per iteration, or null

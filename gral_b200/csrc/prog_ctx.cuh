@@ -76,6 +76,14 @@ struct gral_ctx {
     // strips, then V, W on strip variant 0 (-1: not tuned yet)
     int pmode = -1;
     int fstrip_grid = 0;       // grid of the fused strip launch
+    // row-chain schedule (plain mode 2+strip_num_variants(), model 1): buffers and grids
+    bool chain_ok = false;     // the loaded grid's records and words fit on the device
+    int chain_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // indexed by PH_*
+    ChainBufs cb{};
+    DevBuf<float2> crec;
+    DevBuf<unsigned long long> cwords;
+    DevBuf<float2> cptab;
+    DevBuf<int> cint;          // iteration epoch, flags of the elimination table's passes
     int forced_pmode = -1;     // GRAL_PROG_PLAIN_MODE
     int strip_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // indexed by PH_*
     float ptune_ms[16] = {0};  // autotuner timings per plain mode
@@ -156,6 +164,7 @@ struct gral_ctx {
         meta.release(); cflags.release(); colf.release(); sit.release(); colke.release(); rcw.release();
         ddpm.release(); dtab.release(); ddt.release(); dflags.release(); fseg.release();
         varw.release(); z0i.release();
+        crec.release(); cwords.release(); cptab.release(); cint.release();
         gff.release(); gffoff.release(); gffkk.release(); gffu.release(); l2flush.release();
         prep.release();
         flags.release(); misc.release(); diag.release(); bcl.release(); counts.release();
@@ -177,6 +186,8 @@ int plain_schedule_default(gral_ctx *ctx);
 int strip_variant_of(const gral_ctx *ctx);
 // the loaded plain mode runs pressure..U as one fused strip launch
 bool fused_strips(const gral_ctx *ctx);
+// the loaded plain mode is the row-chain schedule
+bool use_chain(const gral_ctx *ctx);
 
 inline int fail(gral_ctx *c, int code, const std::string &msg) {
     if (c) c->err = msg;

@@ -216,9 +216,14 @@ int validate(gral_ctx *ctx, int n, const gral_params *p, const gral_static *s, c
     return GRAL_OK;
 }
 
+// the plain mode of the row-chain schedule, after the fused strips
+int kChainMode() { return 2 + strip_num_variants(); }
+
 // The slab family's model-1 sweeps run on the strip schedule (pmode 1+v) rather than the
 // diagonal-claim wavefront (pmode 0).
-bool use_strips(const gral_ctx *ctx) { return !ctx->il && ctx->model == 1 && ctx->pmode > 0; }
+bool use_strips(const gral_ctx *ctx) {
+    return !ctx->il && ctx->model == 1 && ctx->pmode > 0 && ctx->pmode < kChainMode();
+}
 
 }  // namespace
 
@@ -230,6 +235,8 @@ bool gral::fused_strips(const gral_ctx *ctx) {
     return use_strips(ctx) && ctx->pmode == 1 + strip_num_variants();
 }
 
+bool gral::use_chain(const gral_ctx *ctx) { return !ctx->il && ctx->model == 1 && ctx->pmode == kChainMode(); }
+
 namespace {
 
 // One SIMPLE iteration (PrognosticFlowfield.cs:584-1182), enqueued on st.
@@ -237,6 +244,16 @@ void launch_iteration(gral_ctx *ctx, cudaStream_t st) {
     const KArgs &a = ctx->ka;
     cudaMemsetAsync(ctx->counters.p, 0, 8 * kCounterSlots * sizeof(unsigned int), st);
     launch_bc(a, ctx->bc, st);
+    if (use_chain(ctx)) {
+        launch_chain(PH_PRESSURE, a, ctx->geo_p.g, ctx->cb, ctx->chain_grid[PH_PRESSURE], st);
+        launch_velcorr(a, st);
+        launch_average(a, st);
+        launch_chain(PH_U, a, ctx->geo_u.g, ctx->cb, ctx->chain_grid[PH_U], st);
+        launch_chain(PH_V, a, ctx->geo_v.g, ctx->cb, ctx->chain_grid[PH_V], st);
+        launch_chain(PH_W, a, ctx->geo_p.g, ctx->cb, ctx->chain_grid[PH_W], st);
+        launch_bookkeeping(a, st);
+        return;
+    }
     if (use_strips(ctx)) {
         const int v = strip_variant_of(ctx);
         if (fused_strips(ctx)) {
@@ -273,6 +290,7 @@ void launch_iteration(gral_ctx *ctx, cudaStream_t st) {
 int launches_per_iteration(const gral_ctx *ctx) {
     const int gs = ctx->ka.group_set <= 0 ? ctx->ngroups : ctx->ka.group_set;
     const int sets = ctx->il ? (ctx->ngroups + gs - 1) / gs : 1;
+    if (use_chain(ctx)) return 3 + 4 * 2 * ((ctx->nb + ctx->cb.unit_n - 1) / ctx->cb.unit_n) + 3;
     if (fused_strips(ctx)) return 3 + 3 + 1;
     if (use_strips(ctx)) return 3 + 4 + 3;
     if (ctx->fused) return 3 + 1 + 2 + 1;
@@ -307,6 +325,14 @@ int size_grids(gral_ctx *ctx) {
         const long long want_blocks = (long long)std::ceil(la * diag_width / (double)warps_per_block);
         if (!il && la > 0) blocks = std::max<long long>(ctx->num_sms, std::min(blocks, want_blocks));
         ctx->grid_gs[kinds[q]] = (int)blocks;
+    }
+    ctx->ka.chain = use_chain(ctx) ? 1 : 0;
+    if (use_chain(ctx)) {
+        const Geom *gk[4] = {&ctx->geo_p, &ctx->geo_u, &ctx->geo_v, &ctx->geo_p};
+        for (int q = 0; q < 4; ++q) {
+            const long long claims = (long long)chain_claims(gk[q]->g.ni) * ctx->cb.unit_n;
+            CK(chain_grid(kinds[q], ctx->ka, claims, &ctx->chain_grid[kinds[q]]));
+        }
     }
     if (use_strips(ctx)) {
         // one block per strip at most: the strip kernels are persistent and claim strips in order
@@ -388,18 +414,22 @@ int tune_variants(gral_ctx *ctx) {
     return build_graph(ctx);
 }
 
-// Autotuner of the slab family (model 1): the diagonal-claim wavefront and every strip variant
-// give bit-identical results, so before the first convergence test each mode runs two live
-// iterations (the first warms the kernels up), the second timed with CUDA events, and the fastest
-// mode is kept and captured into the iteration graph.  Without room for the trials the default
-// mode is kept.
+// Schedule of the slab family's model-1 sweeps.  The row chains are the fastest on every grid measured
+// (ms of an iteration, row chains / best other: 16x14 0.17 / 0.24, 100x100 0.60 / 1.53, 200x200 1.33 /
+// 3.54, 400x400 3.38 / 8.33), so they run wherever their buffers fit.  Otherwise the diagonal-claim
+// wavefront and the strip variants, which give bit-identical results, each run two live iterations
+// before the first convergence test (the first warms the kernels up), the second timed with CUDA
+// events, and the fastest is kept and captured into the iteration graph; without room for the trials
+// the default strip variant is kept.
 constexpr int kDefaultPlainMode = 1;   // strips of 4 rows, 4 warps per row (fastest on the 400x400 grid)
 
 }  // namespace
 
 int gral::plain_schedule_default(gral_ctx *ctx) {
-    const int nv = 2 + strip_num_variants();
-    ctx->pmode = (ctx->model != 1) ? 0 : ((ctx->forced_pmode >= 0 && ctx->forced_pmode < nv) ? ctx->forced_pmode : kDefaultPlainMode);
+    const int nv = kChainMode() + (ctx->chain_ok ? 1 : 0);
+    ctx->pmode = (ctx->model != 1) ? 0
+                 : ((ctx->forced_pmode >= 0 && ctx->forced_pmode < nv) ? ctx->forced_pmode
+                    : (ctx->chain_ok ? kChainMode() : kDefaultPlainMode));
     return size_grids(ctx);
 }
 
@@ -408,11 +438,14 @@ namespace {
 int tune_plain(gral_ctx *ctx) {
     if (ctx->pmode >= 0) return GRAL_OK;
     const int nv = 2 + strip_num_variants();
+    const int forced_nv = kChainMode() + (ctx->chain_ok ? 1 : 0);
     const int first_stop = std::min(((ctx->it_host + ctx->cadence - 1) / ctx->cadence) * ctx->cadence, ctx->it_max);
     if (ctx->model != 1) {
         ctx->pmode = 0;
-    } else if (ctx->forced_pmode >= 0 && ctx->forced_pmode < nv) {
+    } else if (ctx->forced_pmode >= 0 && ctx->forced_pmode < forced_nv) {
         ctx->pmode = ctx->forced_pmode;
+    } else if (ctx->chain_ok) {
+        ctx->pmode = kChainMode();
     } else if (first_stop - ctx->it_host + 1 > 2 * nv) {
         cudaStream_t st = ctx->stream;
         float best = 1e30f;
@@ -471,6 +504,60 @@ int run_diagnostic(gral_ctx *ctx) {
     }
     launch_diag_wfinal(kd, t, st);
     CK(cudaGetLastError());
+    return GRAL_OK;
+}
+
+// Buffers of the row-chain schedule: records for as many situations at a time as fit kChainBytes (the
+// situations are independent, so sets of them run one after the other), the words between strips and
+// the elimination table of the pressure sweep, built here.  If they do not fit on the device the
+// strip schedule, which needs none of them, stays the default.
+constexpr size_t kChainBytes = (size_t)8 << 30;
+
+int reserve_chain(gral_ctx *ctx) {
+    ctx->chain_ok = false;
+    ctx->ka.epoch = nullptr;
+    if (ctx->il || ctx->model != 1) return GRAL_OK;
+    cudaStream_t st = ctx->stream;
+    const size_t unit = chain_record_bytes() * ctx->ncols;
+    const size_t words = chain_unit_words(ctx->nii, ctx->njj);
+    int units = (int)std::max<size_t>(1, std::min<size_t>(ctx->nb, kChainBytes / unit));
+    if (const char *v = std::getenv("GRAL_PROG_CHAIN_UNITS")) units = std::max(1, std::min(units, std::atoi(v)));
+    units = std::max(units, (ctx->nb + kCounterSlots - 1) / kCounterSlots);
+    const size_t had = ctx->cwords.n;
+    const int had_int = (int)ctx->cint.n;
+    constexpr int kPasses = 8;     // flags of the table's passes, reused round by round
+    cudaError_t e = ctx->crec.ensure(unit / sizeof(float2) * units);
+    if (e == cudaSuccess) e = ctx->cwords.ensure(words * ctx->nb);
+    if (e == cudaSuccess) e = ctx->cptab.ensure((size_t)2 * ctx->ncols * ctx->ks);
+    if (e == cudaSuccess) e = ctx->cint.ensure(1 + kPasses);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        ctx->crec.release(); ctx->cwords.release(); ctx->cptab.release();
+        return GRAL_OK;
+    }
+    CK(e);
+    // the epoch only grows within a context, so words of earlier loads never carry a current stamp
+    if (had_int == 0) {
+        const int one = 1;
+        CK(cudaMemcpyAsync(ctx->cint.p, &one, sizeof(int), cudaMemcpyHostToDevice, st));
+    }
+    if (ctx->cwords.n != had) CK(cudaMemsetAsync(ctx->cwords.p, 0, ctx->cwords.n * sizeof(unsigned long long), st));
+    ctx->ka.epoch = ctx->cint.p;
+    ctx->cb = ChainBufs{ctx->crec.p, ctx->cwords.p, ctx->cptab.p, ctx->cint.p, 0, units, 0};
+    CK(cudaMemsetAsync(ctx->cptab.p, 0, (size_t)2 * ctx->ncols * ctx->ks * sizeof(float2), st));
+    // passes of the elimination table until one changes nothing: the first two rounds of passes are
+    // enqueued together, a flag that is still set afterwards asks for more
+    int *flags = ctx->cint.p + 1, last = 1;
+    for (int first = 0; last; first = 1) {
+        int h[kPasses];
+        CK(cudaMemsetAsync(flags, 0, kPasses * sizeof(int), st));
+        if (first) { const int one = 1; CK(cudaMemcpyAsync(flags, &one, sizeof(int), cudaMemcpyHostToDevice, st)); }
+        launch_pressure_tab(ctx->ka, ctx->cptab.p, flags, first, kPasses - first, st);
+        CK(cudaMemcpyAsync(h, flags, sizeof(h), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        last = h[kPasses - 1];
+    }
+    ctx->chain_ok = true;
     return GRAL_OK;
 }
 
@@ -952,6 +1039,8 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
     launch_gather(a, sg, ctx->model, st);
     CK(cudaGetLastError());
 
+    CK_RC(reserve_chain(ctx));
+
     // ---- launch shapes of the wavefront kernels ----
     CK(gs_prepare(il, ks, ctx->model));
     ctx->it_host = 1;
@@ -1013,12 +1102,21 @@ int gral_prog_iterate_timed(gral_ctx *ctx, int32_t iterations, double *phase_ms,
     const KArgs &a = ctx->ka;
     // the iteration's launches in order, each tagged with the phase it is timed under
     std::vector<std::pair<int, std::function<void()>>> seq;
+    const bool chain = use_chain(ctx);
+    auto chain_phase = [&](int kind, const Geom &G) { launch_chain(kind, a, G.g, ctx->cb, ctx->chain_grid[kind], st); };
     seq.push_back({GRAL_PHASE_BC, [&] {
         cudaMemsetAsync(ctx->counters.p, 0, 8 * kCounterSlots * sizeof(unsigned int), st);
         launch_bc(a, ctx->bc, st);
     }});
     const int sv = strip_variant_of(ctx);
-    if (use_strips(ctx)) {
+    if (chain) {
+        seq.push_back({GRAL_PHASE_PRESSURE, [&] { chain_phase(PH_PRESSURE, ctx->geo_p); }});
+        seq.push_back({GRAL_PHASE_VELCORR, [&] { launch_velcorr(a, st); }});
+        seq.push_back({GRAL_PHASE_AVERAGE, [&] { launch_average(a, st); }});
+        seq.push_back({GRAL_PHASE_U, [&] { chain_phase(PH_U, ctx->geo_u); }});
+        seq.push_back({GRAL_PHASE_V, [&] { chain_phase(PH_V, ctx->geo_v); }});
+        seq.push_back({GRAL_PHASE_W, [&] { chain_phase(PH_W, ctx->geo_p); }});
+    } else if (use_strips(ctx)) {
         if (fused_strips(ctx)) {
             seq.push_back({GRAL_PHASE_FUSED, [&] { launch_fused_strip(a, ctx->fgeo, ctx->fstrip_grid, st); }});
         } else {
@@ -1037,7 +1135,7 @@ int gral_prog_iterate_timed(gral_ctx *ctx, int32_t iterations, double *phase_ms,
         seq.push_back({GRAL_PHASE_AVERAGE, [&] { launch_average(a, st); }});
         seq.push_back({GRAL_PHASE_U, [&] { launch_gs(PH_U, a, ctx->geo_u.g, ctx->grid_gs[PH_U], st); }});
     }
-    if (!use_strips(ctx)) {
+    if (!chain && !use_strips(ctx)) {
         seq.push_back({GRAL_PHASE_V, [&] { launch_gs(PH_V, a, ctx->geo_v.g, ctx->grid_gs[PH_V], st); }});
         seq.push_back({GRAL_PHASE_W, [&] { launch_gs(PH_W, a, ctx->geo_p.g, ctx->grid_gs[PH_W], st); }});
     }

@@ -176,6 +176,27 @@ __global__ void k_velcorr(KArgs a) {
     });
 }
 
+// Slab layout after a row-chain pressure sweep: the sweep stores DPM only, so the update of DPMNEW
+// and the residual maximum (:877-893) ride on this pass, which reads DPM anyway.
+__global__ void k_velcorr_press(KArgs a) {
+    col_loop<false>(a, true, [&](int s, int col, int i, int j, const Acc<false> &x, int kbeg, int kstep) {
+        velcorr_col<false>(a, s, col, i, j, x, kbeg, kstep);
+        if (i < 2 || i > a.nii - 1 || j < 2 || j > a.njj - 1 || !(a.cflags[col] & F_ADV)) return;
+        const ColMeta m = a.meta[col];
+        const SitCtx sc = make_sit(a, s);
+        unsigned key = 0;
+        for (int k = kbeg; k <= m.vi; k += kstep) {
+            if (k <= m.kkart) continue;
+            const float temp = a.dpm[x.at(0, k)];
+            key = max(key, residual_key(temp, sc));
+            a.dpmnew[x.at(0, k)] = a.dpmnew[x.at(0, k)] + a.relaxp * temp;
+        }
+        for (int d = 16; d > 0; d >>= 1) key = max(key, __shfl_xor_sync(0xffffffffu, key, d));
+        // one atomic per column at most, and none once the maximum is as large
+        if (kbeg == 0 && key > *(volatile unsigned *)&a.sit[s].dumax_bits) atomicMax(&a.sit[s].dumax_bits, key);
+    });
+}
+
 // ---- staggered -> cell-centre averages and the border copies (:958-1039) ----
 template <bool IL>
 __global__ void k_average(KArgs a) {
@@ -188,7 +209,10 @@ __global__ void k_average(KArgs a) {
 // ---- convergence bookkeeping (:1144-1178), one thread per situation ----
 __global__ void k_bookkeeping(KArgs a) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0) *a.it_global += 1;   // kernels of this launch read SitDev::it, never it_global
+    if (s == 0) {
+        *a.it_global += 1;   // kernels of this launch read SitDev::it, never it_global
+        if (a.epoch) *a.epoch += 1;
+    }
     if (s >= a.nb) return;
     SitDev &S = a.sit[s];
     if (!S.active) return;
@@ -467,7 +491,10 @@ void launch_bc(const KArgs &a, const BcLists &bc, cudaStream_t st) {
     GRAL_COL_LAUNCH(k_bc_top, a);
 }
 
-void launch_velcorr(const KArgs &a, cudaStream_t st) { GRAL_COL_LAUNCH(k_velcorr, a); }
+void launch_velcorr(const KArgs &a, cudaStream_t st) {
+    if (a.chain) k_velcorr_press<<<col_grid<false>(a), COL_WARPS * 32, 0, st>>>(a);
+    else GRAL_COL_LAUNCH(k_velcorr, a);
+}
 
 void launch_average(const KArgs &a, cudaStream_t st) {
     if (a.il) k_average<true><<<col_grid<true, true>(a), COL_WARPS * 32, 0, st>>>(a);

@@ -22,6 +22,17 @@ struct Staging {
     size_t stride;   // floats between situations
 };
 
+// Buffers of the row-chain schedule (prog_chain.cu): column records of the units in flight, stamped
+// words between claims, the pressure sweep's elimination table per i-direction.
+struct ChainBufs {
+    float2 *rec;                 // records [unit][col][pair][KMAX_LEVELS]; pressure: DIV/DTIME [unit][col][KS]
+    unsigned long long *words;   // [situation][claim][column][values][KMAX_LEVELS]
+    const float2 *ptab;          // [dir][col][KS] {T, P}
+    const int *epoch;            // iterations run in this context, part of the word stamps
+    int unit_lo, unit_n;         // situations (positions in the active list) of a launch
+    int ctr_slot;                // task-counter slot of the launch
+};
+
 int gs_num_variants();
 int gs_block_threads(bool il, int variant);
 cudaError_t gs_prepare(bool il, int ks, int model);
@@ -43,6 +54,17 @@ void launch_fused_strip(const KArgs &a, const FusedGeom &fg, int grid, cudaStrea
 // pressure + velocity correction + averages + model-1 U in one wavefront launch (slab family)
 cudaError_t fused_occupancy(int *blocks_per_sm);
 void launch_fused_pvau(const KArgs &a, const FusedGeom &fg, int grid, cudaStream_t st);
+
+// row-chain schedule of the slab family's model-1 sweeps: coefficient launch and chain launch of one
+// phase (kind = PH_PRESSURE, PH_U, PH_V, PH_W); bufs.unit_n situations at a time
+size_t chain_record_bytes();
+size_t chain_unit_words(int nii, int njj);      // words of one unit
+int chain_claims(int ni);                               // claims of a sweep of ni rows
+cudaError_t chain_grid(int kind, const KArgs &a, long long claims, int *grid);
+void launch_chain(int kind, const KArgs &a, const SweepGeom &g, const ChainBufs &bufs, int grid, cudaStream_t st);
+// passes [first, first + passes) of the elimination table; changed[p] (zeroed) says whether pass p
+// changed a value, and the table is complete when its last pass did not
+void launch_pressure_tab(const KArgs &a, float2 *tab, int *changed, int first, int passes, cudaStream_t st);
 
 void launch_bc(const KArgs &a, const BcLists &bc, cudaStream_t st);
 void launch_velcorr(const KArgs &a, cudaStream_t st);
