@@ -75,7 +75,7 @@ struct SitDev {
     int32_t n_hist;
     int32_t it_min, it_max, cadence;
     int32_t quantise;
-    int32_t rcp_ok;          // ConvToInt(x*Frund)/Frund by the reciprocal (verified at the load)
+    int32_t rcp_ok;          // ConvToInt(x*Frund)/Frund by the reciprocal (quantd_r)
 };
 
 // Everything a kernel needs, passed by value (all pointers are device pointers).
@@ -185,11 +185,18 @@ __device__ __forceinline__ int conv_to_int(double v) {
 __device__ __forceinline__ double quantd(double x, double frund, int on) {
     return on ? (double)conv_to_int(x * frund) / frund : x;
 }
-// The same with the division n/Frund (n = ConvToInt(x*Frund), an integer) done as Markstein's
-// correction step on the precomputed y = RN(1/Frund): q0 = RN(n*y), r = n - q0*Frund (exact by
-// FMA), q = RN(q0 + r*y).  rok says that the load-time check (k_rcp_check) found q equal to the
-// IEEE quotient n/Frund for every integer n of magnitude up to 2^31 with this Frund; without it
-// the IEEE division is used.
+// The same with the division n/Frund (n = ConvToInt(x*Frund), an integer of magnitude up to 2^31) done
+// as Markstein's correction step (IBM J. Res. Dev. 34(1), 1990) on the precomputed y = RN(1/Frund):
+// q0 = RN(n*y), r = n - q0*Frund, q = RN(q0 + r*y).  It equals the IEEE quotient for every n because
+// Frund is a float's value, b = B*2^e with B < 2^24:
+//  * q0 is within 1.5 ulp of n/b, so r is a multiple of ulp(q0)*2^e below 2^26 such units: the FMA
+//    gives it exactly;
+//  * q0 + r*y differs from n/b by at most |r/b|*2^-53 <= 1.5*2^-53 ulp, so q can only be wrong if n/b
+//    lies that close to a midpoint m of two doubles.  m = M*2^t with M odd and 2^53 <= M < 2^54:
+//    n = m*b would need M to divide n (M is odd) although M > n, so n/b is no midpoint, and then
+//    |n - m*b| >= 2^(t+e), the unit of both: |n/b - m| >= 2^t/B > 2^(t-24), where 2^t is half an ulp.
+// rok: Frund and y are normal numbers (a non-finite or zero wind speed falls back to the division).
+// Loading a situation used to compare all 2^30 cases instead, 1.6 ms each.
 __device__ __forceinline__ double quantd_r(double x, double frund, double rfrund, bool rok, int on) {
     if (!on) return x;
     const double n = (double)conv_to_int(x * frund);
