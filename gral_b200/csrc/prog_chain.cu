@@ -183,13 +183,17 @@ __device__ __forceinline__ void level_rec(LevelRec &r, const MomPre &p, int IS, 
     }
 }
 
-// Coefficients of one model-1 momentum sweep.  Threads map to (column, level) pairs in the slab's
-// memory order, so loads and record stores are contiguous and no lane idles below KS levels; the
-// forward elimination P_k = B_k*T_k, T_k = 1/(A_k - C_k*P_k-1) then runs with a lane per column
-// (32 independent serial chains per warp) on rows in shared memory.
+// Coefficients of one model-1 momentum sweep.  Threads map to (column, level) pairs of the tile's level
+// range in the slab's memory order, so loads and record stores are contiguous and few lanes idle; then a warp
+// per column runs the forward elimination P_k = B_k*T_k, T_k = 1/(A_k - C_k*P_k-1) like the chain's
+// recurrences (its influence fades by C*P*T a level; a lane per column, level by level, left seven
+// of the block's eight warps waiting).
 template <int COMP, int SW>
-__global__ void __launch_bounds__(CT_THREADS, 3) k_mom1_terms(KArgs a, SweepGeom g, ChainBufs b) {
+__global__ void __launch_bounds__(CT_THREADS, 4) k_mom1_terms(KArgs a, SweepGeom g, ChainBufs b) {
     __shared__ float sA[CT_COLS][KMAX_LEVELS + 1], sB[CT_COLS][KMAX_LEVELS + 1], sC[CT_COLS][KMAX_LEVELS + 1];
+    __shared__ ColCtx s_col[CT_COLS];
+    __shared__ float s_ust[CT_COLS];
+    __shared__ int s_lo, s_n;
     const Tile t = make_tile(a, g, b, COMP == COMP_V);
     if (!t.ok) return;
     constexpr int NP = mom_pairs<COMP, SW>(), TP = tp_pair<COMP>();
@@ -199,22 +203,47 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_mom1_terms(KArgs a, SweepGeom
     const float *F = COMP == COMP_U ? a.uk : (COMP == COMP_V ? a.vk : a.wk);
     constexpr size_t rs = (size_t)NP * KL;     // float2 of a record
     float2 *base = b.rec + ((size_t)t.u * a.ncols + (size_t)(t.i * a.nj2 + t.j0)) * rs;
-    for (int q = threadIdx.x; q < t.nc * ks; q += CT_THREADS) {
-        const int cl = q / ks, k = q - cl * ks;
-        const ColCtx c = make_col(a, t.i, t.j0 + cl);
+    // the columns' constants and wall-law friction velocity once per tile
+    if (threadIdx.x < t.nc) {
+        const ColCtx c = make_col(a, t.i, t.j0 + threadIdx.x);
+        s_col[threadIdx.x] = c;
+        s_ust[threadIdx.x] = (COMP != COMP_W && (c.fl & F_ADV)) ? ml_ustern<false>(a, make_acc<false>(a, t.s, c.col), c) : 0.0f;
+    }
+    // the tile's level range: its full items are (column, level in the range), the others only pass
+    // the field's value on
+    if (threadIdx.x < 32) {
+        __syncwarp();
+        const bool on = threadIdx.x < t.nc && (s_col[threadIdx.x].fl & F_ADV);
+        const int lo = __reduce_min_sync(0xffffffffu, on ? s_col[threadIdx.x].K0 : ks);
+        const int hi = __reduce_max_sync(0xffffffffu, on ? s_col[threadIdx.x].VI : -1);
+        if (threadIdx.x == 0) { s_lo = hi < 0 ? 0 : lo; s_n = hi < 0 ? 0 : hi - lo + 1; }
+    }
+    __syncthreads();
+    constexpr int PP = COMP == COMP_W ? 4 : 7;             // the pair of phi and the flags
+    const int klo = s_lo, nlev = s_n, nrest = ks - nlev;
+    auto pass_on = [&](int cl, int k) {
+        LevelRec r;
+        r.phi = F[make_acc<false>(a, t.s, s_col[cl].col).at(0, k)];
+        r.fl = 0u;
+        base[(size_t)cl * rs + k + PP * KL] = rec_pair<COMP, SW>(r, PP);
+    };
+    for (int q = threadIdx.x; q < t.nc * nrest; q += CT_THREADS) {
+        const int cl = q / nrest, k = q - cl * nrest;
+        pass_on(cl, k < klo ? k : k + nlev);
+    }
+    for (int q = threadIdx.x; q < t.nc * nlev; q += CT_THREADS) {
+        const int cl = q / nlev, k = klo + q - cl * nlev;
+        const ColCtx &c = s_col[cl];
+        if (!(c.fl & F_ADV) || k < c.K0 || k > c.VI) {     // a level the sweep does not change
+            pass_on(cl, k);
+            continue;
+        }
         const Acc<false> x = make_acc<false>(a, t.s, c.col);
         float2 *rec = base + (size_t)cl * rs + k;
         LevelRec r;
-        if (!(c.fl & F_ADV) || k < c.K0 || k > c.VI) {     // a level the sweep does not change
-            r.phi = F[x.at(0, k)];
-            r.fl = 0u;
-            constexpr int PP = COMP == COMP_W ? 4 : 7;
-            rec[PP * KL] = rec_pair<COMP, SW>(r, PP);
-            continue;
-        }
         MomPre p;
-        if (COMP == COMP_U) p = u1_pre<false, SW>(a, x, c, sc, k);
-        else if (COMP == COMP_V) p = v1_pre<false, SW>(a, x, c, sc, k);
+        if (COMP == COMP_U) p = u1_pre<false, SW>(a, x, c, sc, k, s_ust + cl);
+        else if (COMP == COMP_V) p = v1_pre<false, SW>(a, x, c, sc, k, s_ust + cl);
         else p = w1_pre<false, SW>(a, x, c, sc, k);
         sA[cl][k] = p.A; sB[cl][k] = p.B; sC[cl][k] = p.C;
         const float sI = F[x.at((long long)t.IS * c.nj2, k)], sJ = F[x.at((long long)t.JS, k)];
@@ -227,24 +256,29 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_mom1_terms(KArgs a, SweepGeom
             if (n != TP) rec[n * KL] = rec_pair<COMP, SW>(r, n);
     }
     __syncthreads();
-    if (threadIdx.x < t.nc) {
-        const int cl = threadIdx.x, col = t.i * a.nj2 + t.j0 + cl;
-        const ColMeta m = a.meta[col];
-        if (a.cflags[col] & F_ADV) {
-            float P = 0.0f;
-            for (int k = m.kstart; k <= m.vi; ++k) {
-                const float A = sA[cl][k], B = sB[cl][k], C = sC[cl][k];
-                const float T = (k > m.kkart + 1) ? 1.0f / (A - C * P) : 1.0f / A;
-                P = B * T;
-                sA[cl][k] = T;
-                sB[cl][k] = P;
-            }
+    // forward elimination, a warp per column and two levels per lane, in rounds until no bit changes
+    const int lane = threadIdx.x & 31;
+    for (int cl = threadIdx.x >> 5; cl < t.nc; cl += CT_THREADS / 32) {
+        const ColCtx &c = s_col[cl];
+        if (!(c.fl & F_ADV)) continue;
+        const int ka = 2 * lane, kb = ka + 1;
+        const bool inA = ka >= c.K0 && ka <= c.VI, inB = kb >= c.K0 && kb <= c.VI;
+        const float A0 = inA ? sA[cl][ka] : 1.0f, B0 = inA ? sB[cl][ka] : 0.0f;
+        const float A1 = inB ? sA[cl][kb] : 1.0f, B1 = inB ? sB[cl][kb] : 0.0f;
+        const bool qA = inA && ka > c.KK + 1, qB = inB && kb > c.KK + 1;
+        const float C0 = qA ? sC[cl][ka] : 0.0f, C1 = qB ? sC[cl][kb] : 0.0f;
+        float T0 = 1.0f / A0, T1 = 1.0f / A1, P0 = B0 * T0, P1 = B1 * T1, in = 0.0f;
+        if (qB) { T1 = 1.0f / (A1 - C1 * P0); P1 = B1 * T1; }
+        for (;;) {
+            const float nx = __shfl_up_sync(0xffffffffu, P1, 1);
+            const bool more = __any_sync(0xffffffffu, __float_as_uint(nx) != __float_as_uint(in));
+            if (!more) break;
+            in = nx;
+            T0 = 1.0f / (qA ? A0 - C0 * in : A0); P0 = B0 * T0;
+            T1 = 1.0f / (qB ? A1 - C1 * P0 : A1); P1 = B1 * T1;
         }
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < t.nc * ks; q += CT_THREADS) {
-        const int cl = q / ks, k = q - cl * ks;
-        base[(size_t)cl * rs + TP * KL + k] = make_float2(sA[cl][k], sB[cl][k]);
+        float4 *rec = reinterpret_cast<float4 *>(base + (size_t)cl * rs + TP * KL) + lane;
+        if (inA || inB) *rec = make_float4(T0, P0, T1, P1);
     }
 }
 

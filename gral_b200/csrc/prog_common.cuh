@@ -99,6 +99,8 @@ struct KArgs {
     float ustern_fx, building_z0;        // Ustern_factorX, building roughness (k-eps wall laws)
     int model;                           // TurbulenceModel 0, 1, 2
     const float *dzk, *hokart;           // [ks]
+    const float *rdz;                    // [ks] 1/DZK, correctly rounded
+    float rdx, rdy;                      // 1/DXK, 1/DYK, correctly rounded
     const float *app, *abp, *atp;        // pressure coefficients per level [ks]
     const float *veg;                    // [ncols][ks] or null
     // per-situation state

@@ -657,10 +657,11 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
 
     // ---- level tables (float, reference expressions) ----
     const float DXK = p0.dxk, DYK = p0.dyk, AREA = DXK * DYK;
-    std::vector<float> tab(5 * ks, 0.0f);   // dzk, hokart, app, abp, atp
+    std::vector<float> tab(6 * ks, 0.0f);   // dzk, hokart, app, abp, atp, 1/dzk
     for (int k = 0; k < ks; ++k) {
         tab[k] = (k < nk2) ? s->dzk[k] : 0.0f;
         tab[ks + k] = (k < nk2) ? s->hokart[k] : 0.0f;
+        tab[5 * ks + k] = 1.0f / tab[k];
     }
     for (int k = 1; k < ks - 1 && k + 1 < nk2; ++k) {                    // PrognosticFlowfield.cs:857-866
         const float *DZ = s->dzk;
@@ -829,7 +830,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
         CK(ctx->varw.ensure((size_t)n * ncols));
         CK(ctx->z0i.ensure(ncols));
     }
-    CK(ctx->tables.ensure(5 * ks));
+    CK(ctx->tables.ensure(6 * ks));
     CK(ctx->ap0.ensure((size_t)n * ks));
     CK(ctx->sit.ensure(n));
     const size_t flag_units = il ? (size_t)ngroups : (size_t)n;
@@ -864,6 +865,8 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
     a.meta = ctx->meta.p; a.cflags = ctx->cflags.p; a.colf = ctx->colf.p;
     a.dzk = ctx->tables.p; a.hokart = ctx->tables.p + ks;
     a.app = ctx->tables.p + 2 * ks; a.abp = ctx->tables.p + 3 * ks; a.atp = ctx->tables.p + 4 * ks;
+    a.rdz = ctx->tables.p + 5 * ks;
+    a.rdx = 1.0f / DXK; a.rdy = 1.0f / DYK;
     a.veg = has_veg ? ctx->veg.p : nullptr;
     a.sit = ctx->sit.p;
     a.ap0 = ctx->ap0.p;

@@ -114,6 +114,53 @@ __device__ __forceinline__ bool simd16(const KArgs &a) {
     return SW == 0 ? a.simd == 16 : SW == 16;
 }
 
+// Correctly rounded quotients without the compiler's range checks and their branches: with y = RN(1/d),
+// q1 = q0 + (x - d*q0)*y is within an ulp of x/d and RN(q1 + (x - d*q1)*y) is the IEEE quotient
+// (P. Markstein, IBM J. Res. Dev. 34(1), 1990), while no remainder leaves the subnormal range and
+// nothing overflows; a non-finite x gives NaN.  rcp_rn is the reciprocal of a divisor in [2^-27, 2^43):
+// one Newton step on the hardware's approximation, compared with 1/d for every significand at every
+// exponent of that range.  A quotient costs 5 operations, three of a level's faces share a divisor.
+__device__ __forceinline__ float rcp_rn(float d) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+    return fmaf(fmaf(-d, y, 1.0f), y, y);
+}
+__device__ __forceinline__ float quot(float x, float d, float y) {
+    float q = x * y;
+    q = fmaf(fmaf(-d, q, x), y, q);
+    return fmaf(fmaf(-d, q, x), y, q);
+}
+
+// sqrt of a sum of squares; zero is kept off the square root's slow path
+__device__ __forceinline__ float sqrt_pos(float x) {
+    const bool z = x == 0.0f;
+    const float r = sqrtf(z ? 1.0f : x);
+    return z ? 0.0f : r;
+}
+
+// Diffusion conductances of a level's six faces, floored at 1e-4 (U-prognostic-microscale_1.cs:270-300),
+// and the power-law coefficients of its fluxes.  East and west (south and north, top and bottom) share
+// their conductance and its reciprocal except on a border of the sub-domain, where one is the floor.
+struct Faces {
+    float DE, DW, DS, DN, DT, DB;
+    float yE, yW, yS, yN, yT;
+};
+__device__ __forceinline__ Faces make_faces(const KArgs &a, const ColCtx &c, int k, float vmx, float dz, float dxdz,
+                                            float dydz) {
+    constexpr float FLOOR = 0.0001f, YF = 1.0f / 0.0001f;
+    Faces f;
+    const float e = vmaxf(quot(vmx * dydz, a.dxk, a.rdx), FLOOR), s = vmaxf(quot(vmx * dxdz, a.dyk, a.rdy), FLOOR);
+    const float ye = rcp_rn(e), ys = rcp_rn(s);
+    f.DT = vmaxf(quot(vmx * a.areaxy, dz, a.rdz[k]), FLOOR);
+    f.DB = (k > c.KK + 1) ? f.DT : FLOOR;
+    f.yT = rcp_rn(f.DT);
+    f.DS = (c.fl & F_BS) ? FLOOR : s; f.yS = (c.fl & F_BS) ? YF : ys;
+    f.DN = (c.fl & F_BN) ? FLOOR : s; f.yN = (c.fl & F_BN) ? YF : ys;
+    f.DW = (c.fl & F_BW) ? FLOOR : e; f.yW = (c.fl & F_BW) ? YF : ye;
+    f.DE = (c.fl & F_BE) ? FLOOR : e; f.yE = (c.fl & F_BE) ? YF : ye;
+    return f;
+}
+
 // Mixing-length eddy viscosity of level k (U-prognostic-microscale_1.cs:239-268) from the column's
 // U and V at k+1 and k-1; zero at and below KKART+1 (the reference masks those lanes).
 // The Vector512 twins take the height above KKART as HOKART[k] - fma(DZK, 0.5, HOKART[KKART])
@@ -125,11 +172,14 @@ __device__ __forceinline__ float ml_vis(const KArgs &a, const ColCtx &c, int k, 
     const float zs = simd16<SW>(a) ? a.hokart[k] - fmaf(dz, 0.5f, c.hokK) : a.hokart[k] - c.hokK - dz * 0.5f;
     float mixL = vminf(0.071f * zs, 100.0f);
     if (c.cf.cov > 0) mixL *= (1.0f - 0.99f * c.cf.cov);
-    float in = (ukp - ukm) / (2.0f * dz);
+    // a difference below 2^-100 squares to zero whatever its quotient's last bit, and a non-finite one
+    // gives the cap either way
+    const float d2 = 2.0f * dz, r2 = 0.5f * a.rdz[k];
+    float in = quot(ukp - ukm, d2, r2);
     const float DUDZ = in * in;
-    in = (vkp - vkm) / (2.0f * dz);
+    in = quot(vkp - vkm, d2, r2);
     const float DVDZ = in * in;
-    return vminf(mixL * mixL * sqrtf(0.5f * (DUDZ + DVDZ)), 15.0f);
+    return vminf(mixL * mixL * sqrt_pos(0.5f * (DUDZ + DVDZ)), 15.0f);
 }
 
 // Friction velocity of the model-1 wall law at KKART+1 (U-prognostic-microscale_1.cs:419-450).
@@ -172,11 +222,33 @@ struct MomPre {
     float hz;                    // DYK*DZK (U) or DXK*DZK (V)
 };
 
+// The six power-law coefficients.  The Peclet numbers only matter between 2^-27 (below, 1 - 0.1*Pe is 1)
+// and 10 (above, the power law's factor is 0), so the quotients need no care at the ends of the range;
+// a non-finite flux shows in their sum and takes the plain divisions.  The bottom flux is zero where
+// the bottom conductance is the floor, so the top's reciprocal serves both.
+__device__ __forceinline__ void face_coefs(MomPre &r, const Faces &f, bool v512, float FE, float FW, float FS, float FN,
+                                           float FT, float FB) {
+    float pT = fabsf(quot(FT, f.DT, f.yT)), pB = fabsf(quot(FB, f.DT, f.yT));
+    float pE = fabsf(quot(FE, f.DE, f.yE)), pW = fabsf(quot(FW, f.DW, f.yW));
+    float pS = fabsf(quot(FS, f.DS, f.yS)), pN = fabsf(quot(FN, f.DN, f.yN));
+    if (!(pT + pB + pE + pW + pS + pN < 1e30f)) {
+        pT = fabsf(FT / f.DT); pB = fabsf(FB / f.DB); pE = fabsf(FE / f.DE);
+        pW = fabsf(FW / f.DW); pS = fabsf(FS / f.DS); pN = fabsf(FN / f.DN);
+    }
+    r.B = pl1(v512, f.DT, pT, -FT);
+    r.C = pl1(v512, f.DB, pB, FB);
+    r.ae = pl1(v512, f.DE, pE, -FE);
+    r.aw = pl1(v512, f.DW, pW, FW);
+    r.as = pl1(v512, f.DS, pS, FS);
+    r.an = pl1(v512, f.DN, pN, -FN);
+}
+
 // U momentum (U-prognostic-microscale_1.cs:205-470).  All operands of the level are loaded first,
 // unconditionally (every address lies inside the padded grid and levels 0..KS-1), so a level costs
 // one memory round trip; the arithmetic follows in the reference's order.
 template <bool IL, int SW = 0>
-__device__ __forceinline__ MomPre u1_pre(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc, int k) {
+__device__ __forceinline__ MomPre u1_pre(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc, int k,
+                                         const float *ust = nullptr) {
     const long long W = -(long long)c.nj2, E = c.nj2, S = -1, N = 1;
     const bool v512 = simd16<SW>(a);
     const float uk = __ldcg(a.uk + x.at(0, k));
@@ -196,31 +268,15 @@ __device__ __forceinline__ MomPre u1_pre(const KArgs &a, const Acc<IL> &x, const
     const float dxdz = DXK * dz, dydz = DYK * dz;
     const float VIS = ml_vis<SW>(a, c, k, dz, ukp, ukm, vkp, vkm);
     const float vmx = vmaxf(VIS, a.vishmin);
-    float DE = vmx * dydz / DXK;
-    float DW = DE;
-    float DS = vmx * dxdz / DYK;
-    float DN = DS;
-    float DT = vmx * AREA / dz;
-    float DB = (k > c.KK + 1) ? DT : 0.0f;
-    if (c.fl & F_BS) DS = 0.0f;
-    if (c.fl & F_BN) DN = 0.0f;
-    if (c.fl & F_BW) DW = 0.0f;
-    if (c.fl & F_BE) DE = 0.0f;
+    const Faces f = make_faces(a, c, k, vmx, dz, dxdz, dydz);
     const float FE = uks * dydz;
     const float FW = uksW * dydz;
     const float FS = 0.25f * (vksW + vks + vksWS + vksS) * dxdz;
     const float FN = 0.25f * (vksW + vks + vksWN + vksN) * dxdz;
     const float FT = 0.25f * (wksW + wks + wksWT + wksT) * AREA;
     const float FB = (k > c.KK + 1) ? 0.25f * (wksW + wks + wksWB + wksB) * AREA : 0.0f;
-    DE = vmaxf(DE, 0.0001f); DB = vmaxf(DB, 0.0001f); DW = vmaxf(DW, 0.0001f);
-    DS = vmaxf(DS, 0.0001f); DN = vmaxf(DN, 0.0001f); DT = vmaxf(DT, 0.0001f);
     MomPre r;
-    r.B = pl1(v512, DT, fabsf(FT / DT), -FT);
-    r.C = pl1(v512, DB, fabsf(FB / DB), FB);
-    r.ae = pl1(v512, DE, fabsf(FE / DE), -FE);
-    r.aw = pl1(v512, DW, fabsf(FW / DW), FW);
-    r.as = pl1(v512, DS, fabsf(FS / DS), FS);
-    r.an = pl1(v512, DN, fabsf(FN / DN), -FN);
+    face_coefs(r, f, v512, FE, FW, FS, FN, FT, FB);
     r.A = r.B + r.C + r.aw + r.as + r.ae + r.an + ap0;
     const float DDPX = dpW - dp0;
     r.t1 = ap0 * 0.5f * (uksW + uks);
@@ -236,11 +292,11 @@ __device__ __forceinline__ MomPre u1_pre(const KArgs &a, const Acc<IL> &x, const
     if (k >= c.wlo && k <= c.whi) {                       // masked wall term of the chunk, :419-450
         const float in = 0.5f * (uksW + uks), in2 = 0.5f * (vksW + vks);
         const float wh = vmaxf(sqrtf(in * in + in2 * in2), 0.1f);
-        const float Ust = ml_ustern(a, x, c);
+        const float Ust = ust ? *ust : ml_ustern(a, x, c);
         const float m2 = (k == c.KK + 1) ? 1.0f : 0.0f;
         r.w = uk / wh * (Ust * Ust) * AREA * m2;
     }
-    r.vdx = VIS / DXK;
+    r.vdx = quot(VIS, DXK, a.rdx);
     r.hz = dydz;
     if (k >= c.kad) {                                      // extra eddy-viscosity terms, :453-470
         r.e0 = (0.5f * (vksEN + vksN) - 0.5f * (vksN + vksWN)) * dxdz;        // DVDXN
@@ -272,7 +328,8 @@ __device__ __forceinline__ float u1_post(const MomPre &p, const ColCtx &c, int k
 
 // V momentum (V-prognostic-microscale_1.cs:205-488); operands first, as u1_pre.
 template <bool IL, int SW = 0>
-__device__ __forceinline__ MomPre v1_pre(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc, int k) {
+__device__ __forceinline__ MomPre v1_pre(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc, int k,
+                                         const float *ust = nullptr) {
     const long long W = -(long long)c.nj2, E = c.nj2, S = -1, N = 1;
     const bool v512 = simd16<SW>(a);
     const float vk = __ldcg(a.vk + x.at(0, k));
@@ -292,31 +349,15 @@ __device__ __forceinline__ MomPre v1_pre(const KArgs &a, const Acc<IL> &x, const
     const float dxdz = DXK * dz, dydz = DYK * dz;
     const float VIS = ml_vis<SW>(a, c, k, dz, ukp, ukm, vkp, vkm);
     const float vmx = vmaxf(VIS, a.vishmin);
-    float DE = vmx * dydz / DXK;
-    float DW = DE;
-    float DS = vmx * dxdz / DYK;
-    float DN = DS;
-    float DT = vmx * AREA / dz;
-    float DB = (k > c.KK + 1) ? DT : 0.0f;
-    if (c.fl & F_BS) DS = 0.0f;
-    if (c.fl & F_BN) DN = 0.0f;
-    if (c.fl & F_BW) DW = 0.0f;
-    if (c.fl & F_BE) DE = 0.0f;
+    const Faces f = make_faces(a, c, k, vmx, dz, dxdz, dydz);
     const float FE = 0.25f * (uks + uksE + uksS + uksES) * dydz;
     const float FW = 0.25f * (uks + uksW + uksS + uksWS) * dydz;
     const float FS = vksS * dxdz;
     const float FN = vks * dxdz;
     const float FT = 0.25f * (wksS + wks + wksST + wksT) * AREA;
     const float FB = (k > c.KK + 1) ? 0.25f * (wksS + wks + wksSB + wksB) * AREA : 0.0f;
-    DE = vmaxf(DE, 0.0001f); DB = vmaxf(DB, 0.0001f); DW = vmaxf(DW, 0.0001f);
-    DS = vmaxf(DS, 0.0001f); DN = vmaxf(DN, 0.0001f); DT = vmaxf(DT, 0.0001f);
     MomPre r;
-    r.B = pl1(v512, DT, fabsf(FT / DT), -FT);
-    r.C = pl1(v512, DB, fabsf(FB / DB), FB);
-    r.ae = pl1(v512, DE, fabsf(FE / DE), -FE);
-    r.aw = pl1(v512, DW, fabsf(FW / DW), FW);
-    r.as = pl1(v512, DS, fabsf(FS / DS), FS);
-    r.an = pl1(v512, DN, fabsf(FN / DN), -FN);
+    face_coefs(r, f, v512, FE, FW, FS, FN, FT, FB);
     r.A = r.B + r.C + r.aw + r.as + r.ae + r.an + ap0;
     const float DDPY = dpS - dp0;
     r.t1 = ap0 * 0.5f * (vksS + vks);
@@ -332,11 +373,11 @@ __device__ __forceinline__ MomPre v1_pre(const KArgs &a, const Acc<IL> &x, const
     if (k >= c.wlo && k <= c.whi) {                       // :437-467
         const float in = 0.5f * (uksW + uks), in2 = 0.5f * (vksW + vks);
         const float wh = vmaxf(sqrtf(in * in + in2 * in2), 0.1f);
-        const float Ust = ml_ustern(a, x, c);
+        const float Ust = ust ? *ust : ml_ustern(a, x, c);
         const float m2 = (k == c.KK + 1) ? 1.0f : 0.0f;
         r.w = vk / wh * (Ust * Ust) * AREA * m2;
     }
-    r.vdx = VIS / DXK;
+    r.vdx = quot(VIS, DXK, a.rdx);
     r.hz = dxdz;
     if (k >= c.kad) {                                      // :470-488
         const float DUDYE = (0.5f * (uksEN + uksE) - 0.5f * (uksE + uksES)) * dxdz;
@@ -391,31 +432,15 @@ __device__ __forceinline__ MomPre w1_pre(const KArgs &a, const Acc<IL> &x, const
     const float dxdz = DXK * dz, dydz = DYK * dz;
     const float VIS = ml_vis<SW>(a, c, k, dz, ukp, ukm, vkp, vkm);
     const float vmx = vmaxf(VIS, a.vishmin);
-    float DE = vmx * dydz / DXK;
-    float DW = DE;
-    float DS = vmx * dxdz / DYK;
-    float DN = DS;
-    float DT = vmx * AREA / dz;
-    float DB = (k > c.KK + 1) ? DT : 0.0f;
-    if (c.fl & F_BS) DS = 0.0f;
-    if (c.fl & F_BN) DN = 0.0f;
-    if (c.fl & F_BW) DW = 0.0f;
-    if (c.fl & F_BE) DE = 0.0f;
+    const Faces f = make_faces(a, c, k, vmx, dz, dxdz, dydz);
     const float FE = 0.25f * (uks + uksE + uksM + uksEB) * dydz;
     const float FW = 0.25f * (uks + uksW + uksM + uksWB) * dydz;
     const float FS = 0.25f * (vks + vksS + vksM + vksSB) * dxdz;
     const float FN = 0.25f * (vks + vksN + vksM + vksNB) * dxdz;
     const float FT = wks * AREA;
     const float FB = (k > c.KK + 1) ? wksB * AREA : 0.0f;
-    DE = vmaxf(DE, 0.0001f); DB = vmaxf(DB, 0.0001f); DW = vmaxf(DW, 0.0001f);
-    DS = vmaxf(DS, 0.0001f); DN = vmaxf(DN, 0.0001f); DT = vmaxf(DT, 0.0001f);
     MomPre r;
-    r.B = pl1(v512, DT, fabsf(FT / DT), -FT);
-    r.C = pl1(v512, DB, fabsf(FB / DB), FB);
-    r.ae = pl1(v512, DE, fabsf(FE / DE), -FE);
-    r.aw = pl1(v512, DW, fabsf(FW / DW), FW);
-    r.as = pl1(v512, DS, fabsf(FS / DS), FS);
-    r.an = pl1(v512, DN, fabsf(FN / DN), -FN);
+    face_coefs(r, f, v512, FE, FW, FS, FN, FT, FB);
     r.A = r.B + r.C + r.aw + r.as + r.ae + r.an + ap0;
     const float DDPZ = dpB - dp0;
     r.t1 = ap0 * 0.5f * (wksB + wks);
@@ -433,7 +458,7 @@ __device__ __forceinline__ MomPre w1_pre(const KArgs &a, const Acc<IL> &x, const
         const float DVDZS = (0.5f * (vksST + vksS) - 0.5f * (vksS + vksSB)) * dxdz;
         const float DWDZT = (wkT - wk) * AREA;
         const float DWDZB = (wk - wkB) * AREA;
-        r.e0 = VIS / dz * (DUDZE - DUDZW + DVDZN - DVDZS + DWDZT - DWDZB);
+        r.e0 = quot(VIS, dz, a.rdz[k]) * (DUDZE - DUDZW + DVDZN - DVDZS + DWDZT - DWDZB);
     }
     r.phi = wk;
     return r;
