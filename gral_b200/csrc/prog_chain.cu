@@ -282,22 +282,39 @@ __global__ void __launch_bounds__(CT_THREADS, 4) k_mom1_terms(KArgs a, SweepGeom
     }
 }
 
-// Divergence term DIV/DTIME of the pressure sweep, [unit][col][KS].
-__global__ void __launch_bounds__(CT_THREADS) k_pressure_terms(KArgs a, SweepGeom g, ChainBufs b) {
-    const Tile t = make_tile(a, g, b, false);
-    if (!t.ok) return;
-    const int ks = a.ks;
-    const SitCtx sc = make_sit(a, t.s);
-    float *base = reinterpret_cast<float *>(b.rec) + ((size_t)t.u * a.ncols + (size_t)(t.i * a.nj2 + t.j0)) * ks;
-    for (int q = threadIdx.x; q < t.nc * ks; q += CT_THREADS) {
-        const int cl = q / ks, k = q - cl * ks;
-        ColCtx c;
-        c.nj2 = a.nj2; c.i = t.i; c.j = t.j0 + cl;
-        c.col = c.i * a.nj2 + c.j;
-        const ColMeta m = a.meta[c.col];
-        c.KK = m.kkart; c.VI = m.vi;
-        if (!(a.cflags[c.col] & F_ADV) || k <= c.KK || k > c.VI) continue;
-        base[q] = pressure_pre<false>(a, make_acc<false>(a, t.s, c.col), c, sc, k);
+// Divergence term DIV/DTIME of the pressure sweep, [unit][col][KS] (pressure_pre per level).  A thread per
+// level of PT_COLS columns, all operands loaded before a column's flags decide anything.
+constexpr int PT_COLS = 2;
+__global__ void __launch_bounds__(256) k_pressure_terms(KArgs a, ChainBufs b) {
+    const int u = blockIdx.y, k = threadIdx.x, ks = a.ks;
+    if (b.unit_lo + u >= *a.nact) return;
+    const int s = a.act[b.unit_lo + u];
+    const size_t E = (size_t)a.nj2 * ks;
+    float u0[PT_COLS], uE[PT_COLS], v0[PT_COLS], vN[PT_COLS], w0[PT_COLS], wT[PT_COLS];
+    uint32_t fl[PT_COLS];
+    ColMeta m[PT_COLS];
+    int col[PT_COLS];
+    bool in[PT_COLS];
+#pragma unroll
+    for (int q = 0; q < PT_COLS; ++q) {
+        const int c = (blockIdx.x * PT_COLS + q) * blockDim.y + threadIdx.y, i = c / a.nj2, j = c - i * a.nj2;
+        in[q] = i >= 2 && i <= a.nii - 1 && j >= 2 && j <= a.njj - 1;
+        col[q] = in[q] ? c : 2 * a.nj2 + 2;
+        const size_t e = ((size_t)s * a.ncols + col[q]) * ks + k;
+        u0[q] = a.uk[e]; uE[q] = a.uk[e + E]; v0[q] = a.vk[e]; vN[q] = a.vk[e + ks];
+        w0[q] = a.wk[e]; wT[q] = a.wk[e + 1];      // level KS of a column is level 0 of the next
+        fl[q] = a.cflags[col[q]];
+        m[q] = a.meta[col[q]];
+    }
+    const float DXK = a.dxk, DYK = a.dyk, AREA = a.areaxy, dz = a.dzk[k], dt = a.sit[s].dtime, rdt = a.sit[s].rdtime;
+    const bool active = a.sit[s].active != 0;
+    float *out = reinterpret_cast<float *>(b.rec) + (size_t)u * a.ncols * ks + k;
+#pragma unroll
+    for (int q = 0; q < PT_COLS; ++q) {
+        if (!in[q] || !active || !(fl[q] & F_ADV) || k <= m[q].kkart || k > m[q].vi) continue;
+        const float h = (u0[q] - uE[q]) * DYK * dz + (v0[q] - vN[q]) * DXK * dz;
+        const float DIV = (k > m[q].kkart + 1) ? h + (w0[q] - wT[q]) * AREA : h - wT[q] * AREA;
+        out[(size_t)col[q] * ks] = div_by(DIV, dt, rdt);
     }
 }
 
@@ -962,7 +979,6 @@ KFn chain_kernel(int kind, const KArgs &a) {
 KFn terms_kernel(int kind, int simd) {
     const bool w = simd == 16;
     switch (kind) {
-        case PH_PRESSURE: return k_pressure_terms;
         case PH_U: return w ? k_mom1_terms<COMP_U, 16> : k_mom1_terms<COMP_U, 8>;
         case PH_V: return w ? k_mom1_terms<COMP_V, 16> : k_mom1_terms<COMP_V, 8>;
         default: return w ? k_mom1_terms<COMP_W, 16> : k_mom1_terms<COMP_W, 8>;
@@ -1003,7 +1019,12 @@ void launch_chain(int kind, const KArgs &a, const SweepGeom &g, const ChainBufs 
     for (b.unit_lo = 0; b.unit_lo < a.nb; b.unit_lo += bufs.unit_n, ++b.ctr_slot) {
         const int n = std::min(bufs.unit_n, a.nb - b.unit_lo);
         const long long tiles = (long long)n * g.ni * ((g.nj + CT_COLS - 1) / CT_COLS);
-        terms_kernel(kind, a.simd)<<<(unsigned)tiles, CT_THREADS, 0, st>>>(a, g, b);
+        if (kind == PH_PRESSURE) {
+            const int rows = std::max(1, 256 / a.ks), per = rows * PT_COLS;
+            k_pressure_terms<<<dim3((a.ncols + per - 1) / per, n), dim3(a.ks, rows), 0, st>>>(a, b);
+        } else {
+            terms_kernel(kind, a.simd)<<<(unsigned)tiles, CT_THREADS, 0, st>>>(a, g, b);
+        }
         chain_kernel(kind, a)<<<grid, CH_THREADS, 0, st>>>(a, g, b);
     }
 }

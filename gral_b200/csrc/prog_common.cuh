@@ -63,6 +63,7 @@ struct SitDev {
     double hist[MAX_HIST];
     unsigned long long geschw_bits;   // GESCHW_MAX as non-negative double bits (atomicMax)
     float dtime, topwind, ug, vg;
+    float rdtime;            // 1/DTIME correctly rounded (host)
     float potdtdz;           // Program.PotdTdz of the situation (k-eps buoyancy)
     float std_dev_v, v0_1;   // TURB initialisation (PrognosticFlowfield.cs:477-486)
     int32_t turb_init;       // 0: initialise TURB/TDISS as the reference, 1: keep the caller's
@@ -100,6 +101,7 @@ struct KArgs {
     int model;                           // TurbulenceModel 0, 1, 2
     const float *dzk, *hokart;           // [ks]
     const float *rdz;                    // [ks] 1/DZK, correctly rounded
+    const float *rdzz;                   // [ks] 1/(DZK[k] + DZK[k-1]), correctly rounded
     float rdx, rdy;                      // 1/DXK, 1/DYK, correctly rounded
     const float *app, *abp, *atp;        // pressure coefficients per level [ks]
     const float *veg;                    // [ncols][ks] or null

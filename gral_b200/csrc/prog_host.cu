@@ -657,11 +657,12 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
 
     // ---- level tables (float, reference expressions) ----
     const float DXK = p0.dxk, DYK = p0.dyk, AREA = DXK * DYK;
-    std::vector<float> tab(6 * ks, 0.0f);   // dzk, hokart, app, abp, atp, 1/dzk
+    std::vector<float> tab(7 * ks, 0.0f);   // dzk, hokart, app, abp, atp, 1/dzk, 1/(dzk + dzk below)
     for (int k = 0; k < ks; ++k) {
         tab[k] = (k < nk2) ? s->dzk[k] : 0.0f;
         tab[ks + k] = (k < nk2) ? s->hokart[k] : 0.0f;
         tab[5 * ks + k] = 1.0f / tab[k];
+        if (k > 0) tab[6 * ks + k] = 1.0f / (tab[k] + tab[k - 1]);
     }
     for (int k = 1; k < ks - 1 && k + 1 < nk2; ++k) {                    // PrognosticFlowfield.cs:857-866
         const float *DZ = s->dzk;
@@ -735,6 +736,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
         S.rcp_ok = std::isnormal(S.frund) && std::isnormal(S.rfrund) ? 1 : 0;   // Frund is a float's value: see quantd_r
         S.conv_threshold = q.conv_threshold;
         S.dtime = DT;
+        S.rdtime = 1.0f / DT;
         S.topwind = topwind;
         const bool alloc = (cfl[rx * nj2 + ry] & F_ALLOC3) != 0;
         S.ug = alloc ? 0.5f * (rv[0] + rv[4]) : 0.0f;
@@ -830,7 +832,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
         CK(ctx->varw.ensure((size_t)n * ncols));
         CK(ctx->z0i.ensure(ncols));
     }
-    CK(ctx->tables.ensure(6 * ks));
+    CK(ctx->tables.ensure(7 * ks));
     CK(ctx->ap0.ensure((size_t)n * ks));
     CK(ctx->sit.ensure(n));
     const size_t flag_units = il ? (size_t)ngroups : (size_t)n;
@@ -866,6 +868,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
     a.dzk = ctx->tables.p; a.hokart = ctx->tables.p + ks;
     a.app = ctx->tables.p + 2 * ks; a.abp = ctx->tables.p + 3 * ks; a.atp = ctx->tables.p + 4 * ks;
     a.rdz = ctx->tables.p + 5 * ks;
+    a.rdzz = ctx->tables.p + 6 * ks;
     a.rdx = 1.0f / DXK; a.rdy = 1.0f / DYK;
     a.veg = has_veg ? ctx->veg.p : nullptr;
     a.sit = ctx->sit.p;

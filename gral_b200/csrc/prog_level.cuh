@@ -61,7 +61,7 @@ __device__ __forceinline__ ColCtx make_col(const KArgs &a, int i, int j) {
 }
 
 struct SitCtx {
-    float ug, vg, dtime, potdtdz;
+    float ug, vg, dtime, rdtime, potdtdz;
     double frund;
     int quant;
     const float *ap0;
@@ -70,7 +70,7 @@ struct SitCtx {
 __device__ __forceinline__ SitCtx make_sit(const KArgs &a, int s) {
     SitCtx q;
     const SitDev &S = a.sit[s];
-    q.ug = S.ug; q.vg = S.vg; q.dtime = S.dtime; q.potdtdz = S.potdtdz; q.frund = S.frund; q.quant = S.quantise;
+    q.ug = S.ug; q.vg = S.vg; q.dtime = S.dtime; q.rdtime = S.rdtime; q.potdtdz = S.potdtdz; q.frund = S.frund; q.quant = S.quantise;
     q.ap0 = a.ap0 + (size_t)s * a.ks;
     return q;
 }
@@ -129,6 +129,16 @@ __device__ __forceinline__ float quot(float x, float d, float y) {
     float q = x * y;
     q = fmaf(fmaf(-d, q, x), y, q);
     return fmaf(fmaf(-d, q, x), y, q);
+}
+
+// x/d with y = RN(1/d) for any x: the quotient above where its conditions hold, zero as it is, and the
+// plain division for the rest (magnitudes outside 2^-100 .. 2^97, non-finite values).
+__device__ __forceinline__ float div_by(float x, float d, float y) {
+    const unsigned e = __float_as_uint(x) & 0x7f800000u;
+    const bool zero = x == 0.0f;
+    if (!zero && e - 0x0d800000u >= 0x62800000u) return x / d;
+    const float q = quot(x, d, y);
+    return zero ? x : q;
 }
 
 // sqrt of a sum of squares; zero is kept off the square root's slow path
@@ -527,7 +537,7 @@ __device__ __forceinline__ float pressure_pre(const KArgs &a, const Acc<IL> &x, 
         DIV = (u0 - uE) * DYK * dz + (v0 - vN) * DXK * dz + (w0 - wT) * AREA;
     else
         DIV = (u0 - uE) * DYK * dz + (v0 - vN) * DXK * dz - wT * AREA;
-    return DIV / sc.dtime;
+    return div_by(DIV, sc.dtime, sc.rdtime);
 }
 
 // pi, pj: this sweep's DPM of the predecessors (i-IS, j) and (i, j-JS) at level k
@@ -536,7 +546,7 @@ __device__ __forceinline__ float pressure_post_v(const KArgs &a, float t0, int k
     const float dz = a.dzk[k];
     const float si = (IS == 1) ? (pi + 0.0f) : (0.0f + pi);    // DPMim + DPMip
     const float sj = (JS == 1) ? (pj - 0.0f) : (0.0f - pj);    // DPMjm - DPMjp
-    return t0 + si / DXK * DYK * dz + sj / DYK * DXK * dz;
+    return t0 + div_by(si, DXK, a.rdx) * DYK * dz + div_by(sj, DYK, a.rdy) * DXK * dz;
 }
 
 template <bool IL>
@@ -914,11 +924,11 @@ __device__ __forceinline__ void velcorr_col(const KArgs &a, int s, int col, int 
         for (int q = 0; q < CH; ++q) {
             const int k = kb + q * kstep;
             if (k < 1 || k > m.vi) continue;
-            if (du && m.kkm_u < k) a.uk[x.at(0, k)] = (float)quantd_r((double)(u[q] + (dw[q] - d[q]) / DXK * DT), fr, rfr, rok, qz);
-            if (dv && m.kkm_v < k) a.vk[x.at(0, k)] = (float)quantd_r((double)(v[q] + (ds[q] - d[q]) / DYK * DT), fr, rfr, rok, qz);
+            if (du && m.kkm_u < k) a.uk[x.at(0, k)] = (float)quantd_r((double)(u[q] + div_by(dw[q] - d[q], DXK, a.rdx) * DT), fr, rfr, rok, qz);
+            if (dv && m.kkm_v < k) a.vk[x.at(0, k)] = (float)quantd_r((double)(v[q] + div_by(ds[q] - d[q], DYK, a.rdy) * DT), fr, rfr, rok, qz);
             if (m.kkart + 1 < k)
                 a.wk[x.at(0, k)] =
-                    (float)quantd_r((double)(w[q] + (dk[q] - d[q]) / (a.dzk[k] + a.dzk[k - 1]) * 2 * DT), fr, rfr, rok, qz);
+                    (float)quantd_r((double)(w[q] + div_by(dk[q] - d[q], a.dzk[k] + a.dzk[k - 1], a.rdzz[k]) * 2 * DT), fr, rfr, rok, qz);
             else
                 a.wk[x.at(0, k)] = 0;
         }
