@@ -1,42 +1,13 @@
-// prog_chain.cu -- row-chain schedule of the slab family's Gauss-Seidel sweeps.
-//
-// A sweep is two launches.  A parallel kernel evaluates every column's coefficients and sources
-// (all that does not read values the sweep itself changes), runs the forward elimination and writes
-// one contiguous record per column.  The chain kernel then walks the sweep rows i1, a row's columns
-// j1 in order, and passes finished columns on as stamped words (float bits and a stamp in one 8-byte
-// access): through rings in shared memory inside a block and to the next block of the cluster,
-// through global memory from one cluster's claim to the next.
-//
-// What bounds it: the chain of (rows + columns) column steps.  A step's time is two first-order
-// vertical recurrences over about 40 levels, whose every operation is rounded as in the reference.
-// Run one level after the other they take about 20 (back-substitution) and 12 (Q) cycles a level.
-// Here a lane holds levels 2*lane and 2*lane+1 and the warp iterates x_k = f_k(x_k-1) on all
-// levels at once, each round passing values two levels on through one shuffle, until a whole round
-// changes no bit.  A state that f maps to itself, starting from the exact first level, is the
-// sequential recurrence's result bit for bit (by induction over the levels), whatever the number of
-// rounds; the recurrences are contractions (the influence of a level fades by relax*P <= 0.1 or
-// by C*T, well below 1), so a few rounds reach it instead of forty levels.
-//
-// A claim (the strips of one cluster) is taken from an atomic counter in order and waits only on the
-// claim before, so clusters need not be resident together; the blocks of a cluster are.  Every wait
-// is bounded and gives up when another warp has set the error word.
+// prog_chain.cu -- row chains of the pressure correction and the model-1 momentum sweeps, and the
+// launches of the schedule (prog_chain.cuh).
 #include <algorithm>
 #include <cmath>
 
-#include "prog_common.cuh"
-#include "prog_kernels.cuh"
-#include "prog_level.cuh"
+#include "prog_chain.cuh"
 
 namespace gral {
 
 namespace {
-
-constexpr int CH_RING = 8;    // hand-off slots between a row and the row below it in the block
-constexpr int CH_AHEAD = 4;   // columns of a warp whose records are asked into L2 ahead
-constexpr int CT_COLS = 32;   // columns of a tile of the coefficient kernels
-constexpr int CT_THREADS = 256;
-
-enum { COMP_U = 0, COMP_V = 1, COMP_W = 2 };
 
 // A column record of the momentum sweeps: pairs of values per level, [pair][KMAX_LEVELS] float2, so
 // that a lane reads its two levels of a pair with one 16-byte load at a constant offset (levels from
@@ -48,13 +19,6 @@ __host__ __device__ constexpr int mom_pairs() { return COMP == COMP_W ? 7 : ((CO
 constexpr int MOM_PAIRS_MAX = 10;
 // level flags of a record (bits of a float)
 enum : unsigned { L_Q = 1u, L_U = 2u, L_X = 4u, L_VEG = 8u };
-
-__device__ __forceinline__ void chain_dir(int it, int &IS, int &JS) {
-    // PrognosticFlowfield.cs:770-802
-    const int m = it % 4;
-    IS = (m == 0 || m == 1) ? -1 : 1;
-    JS = (m == 1 || m == 2) ? -1 : 1;
-}
 
 // What a chain step needs of one level: the sums of DIM in the reference's order, split into the
 // parts the predecessors enter (see MomChain::dim).
@@ -121,30 +85,6 @@ template <int COMP>
 __host__ __device__ constexpr int tp_pair() { return COMP == COMP_W ? 6 : 8; }   // the pair that holds T and P
 
 // ------------------------------------ coefficients ------------------------------------------
-
-// Tile of a coefficient launch: CT_COLS columns along j of one sweep row of one unit.
-struct Tile {
-    int u, s, i, j0, nc, IS, JS;
-    bool ok;
-};
-__device__ __forceinline__ Tile make_tile(const KArgs &a, const SweepGeom &g, const ChainBufs &b, bool reverse) {
-    Tile t;
-    chain_dir(*a.it_global, t.IS, t.JS);
-    if (reverse) { t.IS = -t.IS; t.JS = -t.JS; }
-    const int per = (g.nj + CT_COLS - 1) / CT_COLS;
-    const int q = blockIdx.x / per;
-    const int c0 = (blockIdx.x - q * per) * CT_COLS;
-    t.u = q / g.ni;
-    const int i1 = g.ia + (q - t.u * g.ni);
-    t.i = (t.IS == 1) ? i1 : a.nii - i1 + 1;
-    t.nc = min(CT_COLS, g.nj - c0);
-    // the tile's columns in ascending j: sweep columns j1 = ja + c0 ... of either direction
-    t.j0 = (t.JS == 1) ? g.ja + c0 : a.njj - (g.ja + c0 + t.nc - 1) + 1;
-    t.ok = b.unit_lo + t.u < *a.nact;
-    t.s = t.ok ? a.act[b.unit_lo + t.u] : 0;
-    t.ok = t.ok && a.sit[t.s].active;
-    return t;
-}
 
 // The record of one level from its coefficients: products and sums that involve only the successors'
 // old values are formed here, each where the reference's association order allows it.
@@ -349,92 +289,11 @@ __global__ void __launch_bounds__(128) k_pressure_tab(KArgs a, float2 *tab, int 
 
 // ------------------------------------ row chains --------------------------------------------
 
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-// Stamped words of two neighbouring levels.
-struct Words2 {
-    unsigned long long a, b;
-};
-__device__ __forceinline__ unsigned long long word(float v, unsigned stamp) {
-    return ((unsigned long long)stamp << 32) | __float_as_uint(v);
-}
-__device__ __forceinline__ float word_val(unsigned long long w) { return __uint_as_float((unsigned)w); }
-__device__ __forceinline__ bool stamped(const Words2 &w, unsigned stamp) {
-    return (unsigned)(w.a >> 32) == stamp && (unsigned)(w.b >> 32) == stamp;
-}
-// The accesses of a lane without levels (`on` false) are predicated off rather than branched over:
-// a branch costs the chain a reconvergence.
-__device__ __forceinline__ Words2 ld_words(const unsigned long long *p, bool on) {
-    Words2 w;
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.u64 %0, 0;\n\tmov.u64 %1, 0;\n\t"
-        "@q ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];\n\t}"
-        : "=&l"(w.a), "=&l"(w.b)
-        : "l"(p), "r"((unsigned)on)
-        : "memory");
-    return w;
-}
-__device__ __forceinline__ void st_words(unsigned long long *p, const Words2 &w, bool on) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};\n\t}" ::"l"(p),
-        "l"(w.a), "l"(w.b), "r"((unsigned)on)
-        : "memory");
-}
-__device__ __forceinline__ void st_pair(float2 *p, float2 v, bool on) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q st.global.cg.v2.f32 [%0], {%1, %2};\n\t}" ::"l"(p),
-                 "f"(v.x), "f"(v.y), "r"((unsigned)on)
-                 : "memory");
-}
-__device__ __forceinline__ Words2 lds_words(unsigned p) {
-    Words2 w;
-    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(w.a), "=l"(w.b) : "r"(p) : "memory");
-    return w;
-}
-__device__ __forceinline__ void sts_words(unsigned p, const Words2 &w) {
-    asm volatile("st.volatile.shared.v2.u64 [%0], {%1, %2};" ::"r"(p), "l"(w.a), "l"(w.b) : "memory");
-}
-__device__ __forceinline__ void l2_ahead(const void *p, bool on) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q prefetch.global.L2 [%0];\n\t}" ::"l"(p),
-                 "r"((unsigned)on));
-}
-// d = a + b or a * b where `on`, as one predicated instruction: the compiler's own forms of a
-// conditional assignment (a select after the operation, or a branch over it) lengthen the recurrences
-// (a round of the momentum step took 109 cycles with `if`, 80 with a select, 68 this way).
-__device__ __forceinline__ void add_if(float &d, float a, float b, unsigned on) {
-    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q add.rn.f32 %0, %1, %2;\n\t}" : "+f"(d) : "f"(a), "f"(b), "r"(on));
-}
-__device__ __forceinline__ void mul_if(float &d, float a, float b, unsigned on) {
-    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q mul.rn.f32 %0, %1, %2;\n\t}" : "+f"(d) : "f"(a), "f"(b), "r"(on));
-}
-__device__ __forceinline__ bool differ(float a, float b) { return __float_as_uint(a) != __float_as_uint(b); }
-
-// Bound of a spin: every 32nd call looks at the error word and the clock; true when the wait must
-// end (warp-uniform).
-struct SpinBound {
-    unsigned long long t0 = 0;
-    unsigned n = 0;
-    __device__ __forceinline__ bool expired(const KArgs &a) {
-        if (n == 0) t0 = globaltimer_ns();
-        if ((++n & 31) != 0) return false;
-        bool stop = *(volatile int *)a.err != ERR_NONE;
-        if (!stop && globaltimer_ns() - t0 > a.wait_limit_ns) {
-            atomicCAS(a.err, ERR_NONE, ERR_TIMEOUT);
-            stop = true;
-        }
-        return __any_sync(0xffffffffu, stop);
-    }
-};
-
-// Rounds of the two recurrences before the first test; a failed test continues round by round.  One
-// round less or more: 400x400 U chain 0.45 / 0.42 / 0.45 ms for 4 / 3 / 2, pressure 0.58 / 0.57 / 0.60 for
-// 5 / 6 / 4 (the pressure's influence fades by 0.17 a level where the layers are as thick as wide).
-constexpr int ROUNDS_MOM = 3, ROUNDS_PRESS = 6;
-
 // Model-1 momentum: record of one column in registers (two levels per lane) and the step, for one
 // sweep direction (branches on it would stall the chain).
 template <int COMP, int SW, int IS, int JS>
 struct MomChain {
-    static constexpr int NV = 1;                    // values handed to the row below
+    static constexpr int NV = 1, NJ = 1, NF = 1;    // see run_chain
     static constexpr int NP = mom_pairs<COMP, SW>();
     struct Rec {
         float4 f[NP];      // {x(2l), y(2l), x(2l+1), y(2l+1)} of each pair
@@ -444,14 +303,14 @@ struct MomChain {
     };
     float relax;
     float2 hz;
-    float *F;
+    float *F[NF];
     const float4 *rec;     // this lane's part of the next record to load
     const char *line;      // this lane's 128-byte line of the next record to ask into L2
     bool on0, on1;         // whether the line exists (and the one 32 lines on)
 
     __device__ __forceinline__ void init(const KArgs &a, int lane) {
         relax = a.relax;
-        F = COMP == COMP_U ? a.uk : (COMP == COMP_V ? a.vk : a.wk);
+        F[0] = COMP == COMP_U ? a.uk : (COMP == COMP_V ? a.vk : a.wk);
         const float face = COMP == COMP_U ? a.dyk : a.dxk;
         const int l = min(lane, a.ks / 2 - 1);
         hz = make_float2(face * a.dzk[2 * l], face * a.dzk[2 * l + 1]);
@@ -460,7 +319,7 @@ struct MomChain {
     }
     int step_rec;          // float4 to this warp's next record
     template <int M>
-    __device__ __forceinline__ void begin(const KArgs &a, const ChainBufs &b, int u, int col, int lane) {
+    __device__ __forceinline__ void begin(const KArgs &a, const ChainBufs &b, int u, int, int col, int lane) {
         step_rec = JS * M * (NP * (KMAX_LEVELS / 2));
         const float2 *p = b.rec + ((size_t)u * a.ncols + col) * (NP * KMAX_LEVELS);
         rec = reinterpret_cast<const float4 *>(p) + min(lane, a.ks / 2 - 1);
@@ -480,7 +339,7 @@ struct MomChain {
     // the field's values of a column that this sweep does not change
     __device__ __forceinline__ Val still(const KArgs &a, size_t base, int lane) const {
         Val o;
-        o.v[0] = __ldcg(reinterpret_cast<const float2 *>(F + base) + min(lane, a.ks / 2 - 1));
+        o.v[0] = __ldcg(reinterpret_cast<const float2 *>(F[0] + base) + min(lane, a.ks / 2 - 1));
         return o;
     }
     // DIM of one level: the neighbour products and sources in the reference's association order
@@ -525,14 +384,14 @@ struct MomChain {
         add_if(D, D, r.vdx * X, r.fl & L_X);
         return D;
     }
-    __device__ __forceinline__ Val step(const Rec &rc, const Val &vI, const float2 &vJ) const {
+    __device__ __forceinline__ Val step(const Rec &rc, const Val &vI, const float2 (&vJ)[NJ]) const {
         LevelRec A, B;
 #pragma unroll
         for (int q = 0; q < NP; ++q) {
             rec_unpair<COMP, SW>(A, q, make_float2(rc.f[q].x, rc.f[q].y));
             rec_unpair<COMP, SW>(B, q, make_float2(rc.f[q].z, rc.f[q].w));
         }
-        const float Da = dim(A, hz.x, vI.v[0].x, vJ.x), Db = dim(B, hz.y, vI.v[0].y, vJ.y);
+        const float Da = dim(A, hz.x, vI.v[0].x, vJ[0].x), Db = dim(B, hz.y, vI.v[0].y, vJ[0].y);
         // Q_k = D_k*T_k up to KKART+1, above it Q_k = (D_k + C_k*Q_k-1)*T_k
         const unsigned qA = A.fl & L_Q, qB = B.fl & L_Q, uA = A.fl & L_U, uB = B.fl & L_U;
         float Qa = Da * A.T, Qb = Db * B.T, inQ = 0.0f, inU = 0.0f;
@@ -583,7 +442,7 @@ struct MomChain {
 // therefore travels along i with the DPM.  DPMNEW and the residual follow in the velocity correction.
 template <int IS, int JS, bool P2>
 struct PressChain {
-    static constexpr int NV = 2;
+    static constexpr int NV = 2, NJ = 1, NF = 1;
     struct Rec {
         float4 tp;      // {T, P} of the two levels
         float2 d;       // DIV/DTIME
@@ -593,7 +452,7 @@ struct PressChain {
     };
     float2 atp, dz;
     float dxk, dyk, rx, ry;
-    float *F;
+    float *F[NF];
     const float2 *div;
     const float4 *tab;
     const char *line;
@@ -602,7 +461,7 @@ struct PressChain {
     bool on0;
 
     __device__ __forceinline__ void init(const KArgs &a, int lane) {
-        F = a.dpm;
+        F[0] = a.dpm;
         dxk = a.dxk; dyk = a.dyk;
         rx = 1.0f / dxk; ry = 1.0f / dyk;
         const int l = min(lane, a.ks / 2 - 1);
@@ -610,7 +469,7 @@ struct PressChain {
         dz = make_float2(a.dzk[2 * l], a.dzk[2 * l + 1]);
     }
     template <int M>
-    __device__ __forceinline__ void begin(const KArgs &a, const ChainBufs &b, int u, int col, int lane) {
+    __device__ __forceinline__ void begin(const KArgs &a, const ChainBufs &b, int u, int, int col, int lane) {
         hstep = JS * M * (a.ks / 2);
         const int l = min(lane, a.ks / 2 - 1);
         const float *d = reinterpret_cast<const float *>(b.rec) + ((size_t)u * a.ncols + col) * a.ks;
@@ -646,10 +505,10 @@ struct PressChain {
         const float qi = P2 ? si * rx : si / dxk, qj = P2 ? sj * ry : sj / dyk;
         return t0 + qi * dyk * dzk + qj * dxk * dzk;
     }
-    __device__ __forceinline__ Val step(const Rec &r, const Val &vI, const float2 &vJ) const {
+    __device__ __forceinline__ Val step(const Rec &r, const Val &vI, const float2 (&vJ)[NJ]) const {
         const float Ta = r.tp.x, Pa = r.tp.y, Tb = r.tp.z, Pb = r.tp.w;
         const unsigned lA = Ta != 0.0f, lB = Tb != 0.0f;
-        const float Da = dim(r.d.x, dz.x, vI.v[0].x, vJ.x), Db = dim(r.d.y, dz.y, vI.v[0].y, vJ.y);
+        const float Da = dim(r.d.x, dz.x, vI.v[0].x, vJ[0].x), Db = dim(r.d.y, dz.y, vI.v[0].y, vJ[0].y);
         // Q downwards from the carry at VerticalIndex+1
         float Qa = vI.v[1].x, Qb = vI.v[1].y, inQ = 0.0f, inD = 0.0f;
         mul_if(Qb, Db, Tb, lB);
@@ -694,236 +553,6 @@ struct PressChain {
     }
 };
 
-// Bytes of a ring slot (every lane's words of one column) and of a ring in shared memory.
-template <int NV>
-__host__ __device__ constexpr unsigned slot_bytes() { return NV * 32u * 16u; }
-template <int NV>
-__host__ __device__ constexpr unsigned ring_bytes() { return CH_RING * slot_bytes<NV>(); }
-
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-// address of this block's shared-memory location p in block `rank` of the cluster
-__device__ __forceinline__ unsigned remote(unsigned p, unsigned rank) {
-    unsigned q;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(q) : "r"(p), "r"(rank));
-    return q;
-}
-__device__ __forceinline__ void st_remote(unsigned p, const Words2 &w, bool on) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};\n\t}" ::"r"(p),
-        "l"(w.a), "l"(w.b), "r"((unsigned)on)
-        : "memory");
-}
-__device__ __forceinline__ void st_remote(unsigned p, int v, bool on) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.relaxed.cluster.shared::cluster.s32 [%0], %1;\n\t}" ::"r"(p),
-                 "r"(v), "r"((unsigned)on)
-                 : "memory");
-}
-__device__ __forceinline__ unsigned ld_remote(unsigned p) {
-    unsigned v;
-    asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
-    return v;
-}
-
-// Shared memory of a block: the rings 0..SR (ring r: what row r takes from above; ring SR: what the
-// strip's last row finished), the claim, and how many columns each ring's reader has taken.
-template <int SR, int NV>
-struct ChainSmem {
-    alignas(16) unsigned long long ring[(SR + 1) * ring_bytes<NV>() / 8];
-    unsigned claim;
-    int taken[SR + 1];
-};
-
-// One cluster of CL blocks takes CL strips of SR rows each (a claim), M warps per row: warp m of a
-// row runs the columns m, m+M, ..., so that while one warp is in its step the row's other warps
-// store, ask for their next record and load it.  A finished column goes into the ring of the row
-// below, where that row and the next column's warp of this row read it; from the last row of a
-// strip also into ring 0 of the next block of the cluster, and from the last row of the claim into
-// the words in global memory, which the feeder warp of the next claim's first block turns into its
-// ring 0 (for the sweep's first row: the values the sweep does not change).
-template <class Job, int PH, int SR, int M, int CL, int IS, int JS>
-__device__ __forceinline__ void run_chain(const KArgs &a, const SweepGeom &g, const ChainBufs &b,
-                                          ChainSmem<SR, Job::NV> &sm) {
-    constexpr int NV = Job::NV;
-    constexpr int WCOL = NV * KMAX_LEVELS;        // words of a column in global memory
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ks = a.ks, nj = g.nj, l2 = 2 * lane;
-    const bool mine = l2 < ks;       // this lane holds levels of the column
-    const unsigned rank = cluster_rank();
-    const unsigned ring0 = smem_u32(sm.ring) + lane * 16u;
-    Job job;
-    job.init(a, lane);
-    const unsigned gstamp = (unsigned)*b.epoch * 8u + PH;      // of the words in global memory
-    const unsigned units = (unsigned)min(b.unit_n, max(0, *a.nact - b.unit_lo));
-    const unsigned ngroups = (unsigned)((g.ni + SR * CL - 1) / (SR * CL));
-    const unsigned total = ngroups * units;
-    unsigned *ctr = a.counters + 8 * b.ctr_slot + PH;
-    unsigned seq = 0;                // claims run by this block: part of the ring stamps
-    const int jfirst = (JS == 1) ? g.ja : a.njj - g.ja + 1;
-    const size_t wrow = (size_t)nj * WCOL;
-    for (;;) {
-        cluster_sync();
-        if (rank == 0 && threadIdx.x == 0)
-            sm.claim = (*(volatile int *)a.err != ERR_NONE) ? 0xffffffffu : atomicAdd(ctr, 1u);
-        if (threadIdx.x <= SR) sm.taken[threadIdx.x] = 0;
-        cluster_sync();
-        const unsigned t = ld_remote(remote(smem_u32(&sm.claim), 0));
-        if (t >= total) break;
-        ++seq;
-        const int u = (int)(t % units), group = (int)(t / units);
-        const int s = a.act[b.unit_lo + u];
-        const int first = g.ia + (group * CL + (int)rank) * SR, rows = min(SR, g.ia + g.ni - first);
-        if (!a.sit[s].active || rows <= 0) continue;
-        auto row_i = [&](int r) { return (IS == 1) ? first + r : a.nii - (first + r) + 1; };
-        unsigned long long *gout = b.words + ((size_t)(b.unit_lo + u) * ngroups + group) * wrow + l2;
-        const unsigned sbase = seq << 16;
-        // waits until ring r's reader has taken n columns (their slots are free)
-        int seen = 0;
-        auto room = [&](int r, int n) {
-            if (seen >= n) return true;
-            SpinBound sb;
-            for (;;) {
-                seen = __shfl_sync(0xffffffffu, *(volatile int *)(sm.taken + r), 0);
-                if (seen >= n) return true;
-                if (sb.expired(a)) return false;
-            }
-        };
-        auto slot = [&](int c) { return (unsigned)(c & (CH_RING - 1)) * slot_bytes<NV>(); };
-        auto push = [&](unsigned ring, int c, const typename Job::Val &v) {
-            const unsigned st = sbase + (unsigned)(c + 1), p = ring + slot(c);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) sts_words(p + q * 512u, Words2{word(v.v[q].x, st), word(v.v[q].y, st)});
-        };
-        if (warp == SR * M) {                                      // the feeder
-            constexpr int NF = 4;                                  // columns in flight
-            bool ok = true;
-            if (rank > 0) {
-            } else if (group > 0) {
-                const unsigned long long *gin = gout - wrow;
-                Words2 w[NF][NV];
-                auto peek = [&](int c, Words2 (&x)[NV]) {
-#pragma unroll
-                    for (int q = 0; q < NV; ++q) x[q] = ld_words(gin + (size_t)c * WCOL + q * KMAX_LEVELS, mine && c < nj);
-                };
-                auto feed = [&](int c, Words2 (&x)[NV]) {
-                    SpinBound sb;
-                    for (;;) {
-                        bool got = true;
-#pragma unroll
-                        for (int q = 0; q < NV; ++q) got = got && stamped(x[q], gstamp);
-                        if (__all_sync(0xffffffffu, got || !mine)) break;
-                        if (sb.expired(a)) return false;
-                        peek(c, x);
-                    }
-                    typename Job::Val v;
-#pragma unroll
-                    for (int q = 0; q < NV; ++q) v.v[q] = make_float2(word_val(x[q].a), word_val(x[q].b));
-                    if (!room(0, c - CH_RING + 1)) return false;
-                    push(ring0, c, v);
-                    peek(c + NF, x);
-                    return true;
-                };
-#pragma unroll
-                for (int q = 0; q < NF; ++q) peek(q, w[q]);
-                for (int c = 0; c < nj && ok; c += NF)
-#pragma unroll
-                    for (int q = 0; q < NF; ++q)
-                        if (ok && c + q < nj) ok = feed(c + q, w[q]);
-            } else {
-                const int cb = (row_i(0) - IS) * a.nj2 + jfirst;
-                auto value = [&](int c) {
-                    return job.still(a, ((size_t)s * a.ncols + (size_t)(cb + JS * min(c, nj - 1))) * ks, lane);
-                };
-                typename Job::Val v[NF];
-#pragma unroll
-                for (int q = 0; q < NF; ++q) v[q] = value(q);
-                for (int c = 0; c < nj && ok; c += NF)
-#pragma unroll
-                    for (int q = 0; q < NF; ++q)
-                        if (ok && c + q < nj) {
-                            ok = room(0, c + q - CH_RING + 1);
-                            push(ring0, c + q, v[q]);
-                            v[q] = value(c + q + NF);
-                        }
-            }
-            continue;
-        }
-        const int r = warp / M, m = warp - r * M;
-        if (r >= rows) continue;
-        const bool more_rows = first + rows < g.ia + g.ni;             // a strip follows this one
-        const bool last = r + 1 == rows;                               // the strip's last row
-        const bool next_block = last && more_rows && rank + 1 < CL;    // ... read by the cluster's next block
-        const bool next_claim = last && more_rows && rank + 1 == CL && mine;
-        const unsigned ring_in = ring0 + (unsigned)r * ring_bytes<NV>(), ring_out = ring_in + ring_bytes<NV>();
-        const unsigned ring_far = remote(ring0, min(rank + 1, CL - 1u));
-        const unsigned taken_far = remote(smem_u32(sm.taken + SR), max((int)rank, 1) - 1);
-        const bool far_above = r == 0 && rank > 0 && lane == 0;        // this row reads the block before
-        const bool watch = !last || next_block;                        // somebody reads this row's columns
-        const int taker = last ? SR : r + 1;
-        const int col0 = row_i(r) * a.nj2 + jfirst;
-        const size_t e0 = ((size_t)s * a.ncols + (size_t)col0) * ks;
-        float2 *out_f = reinterpret_cast<float2 *>(job.F + e0) + lane + (long long)m * JS * (ks / 2);
-        unsigned long long *wout = gout + (size_t)m * WCOL;
-        job.template begin<M>(a, b, u, col0 + JS * m, lane);
-        if (m == 0) push(ring_out, -1, job.still(a, e0 - (long long)JS * ks, lane));   // left of the first column
-        typename Job::Rec rec;
-        for (int c = m; c < m + CH_AHEAD * M; c += M) job.ahead(c < nj);
-        if (m < nj) job.load(rec);
-        for (int c = m; c < nj; c += M) {
-            Words2 wI[NV], wJ;
-            const unsigned want = sbase + (unsigned)(c + 1), pI = ring_in + slot(c), pJ = ring_out + slot(c - 1);
-            SpinBound sb;
-            bool ok = true;
-            for (;;) {
-                wJ = lds_words(pJ);
-#pragma unroll
-                for (int q = 0; q < NV; ++q) wI[q] = lds_words(pI + q * 512u);
-                bool got = stamped(wJ, want - 1u);
-#pragma unroll
-                for (int q = 0; q < NV; ++q) got = got && stamped(wI[q], want);
-                if (__all_sync(0xffffffffu, got)) break;
-                if (sb.expired(a)) { ok = false; break; }
-            }
-            typename Job::Val vI;
-#pragma unroll
-            for (int q = 0; q < NV; ++q) vI.v[q] = make_float2(word_val(wI[q].a), word_val(wI[q].b));
-            const typename Job::Val v = job.step(rec, vI, make_float2(word_val(wJ.a), word_val(wJ.b)));
-            if (!ok) break;
-            push(ring_out, c, v);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                const unsigned st = sbase + (unsigned)(c + 1);
-                st_remote(ring_far + slot(c) + q * 512u, Words2{word(v.v[q].x, st), word(v.v[q].y, st)}, next_block);
-            }
-            // the rest runs while the row's next column is in its step
-            *(volatile int *)(sm.taken + r) = c + 1;
-            st_remote(taken_far, c + 1, far_above);
-            if (c + M < nj) job.load(rec);
-#pragma unroll
-            for (int q = 0; q < NV; ++q)
-                st_words(wout + q * KMAX_LEVELS, Words2{word(v.v[q].x, gstamp), word(v.v[q].y, gstamp)}, next_claim);
-            st_pair(out_f, v.v[0], mine);     // levels the sweep does not change keep their value
-            wout += (size_t)M * WCOL;
-            out_f += M * JS * (ks / 2);
-            job.ahead(c + CH_AHEAD * M < nj);
-            if (watch && !room(taker, c + M - CH_RING + 1)) break;
-        }
-    }
-    cluster_sync();      // no block leaves while another may still write into its shared memory
-}
-
-// Strip shape: rows of a block, warps of a row, blocks of a cluster.  Measured on the 400x400 grid,
-// ms of an iteration: (4,2,8) 3.44, (3,2,8) 3.51, (2,3,8) 3.61, (4,3,8) 3.48; one warp per row and every
-// hand-off between blocks through global memory 4.25.
-constexpr int CH_SR = 4, CH_M = 2, CH_CL = 8;
-constexpr int CH_THREADS = (CH_SR * CH_M + 1) * 32;
-
 // The kernels take the sweep's direction from the iteration count and run the code built for it.
 template <int COMP, int SW>
 __global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 1) k_mom_chain(KArgs a, SweepGeom g, ChainBufs b) {
@@ -959,7 +588,6 @@ __global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 1) k
     }
 }
 
-using KFn = void (*)(KArgs, SweepGeom, ChainBufs);
 
 bool pow2(float x) {
     int e;
@@ -968,6 +596,7 @@ bool pow2(float x) {
 
 KFn chain_kernel(int kind, const KArgs &a) {
     const bool w = a.simd == 16;
+    if (kind != PH_PRESSURE && a.model != 1) return chain_scalar_kernel(kind, a.model);
     switch (kind) {
         case PH_PRESSURE: return (pow2(a.dxk) && pow2(a.dyk)) ? k_pressure_chain<true> : k_pressure_chain<false>;
         case PH_U: return w ? k_mom_chain<COMP_U, 16> : k_mom_chain<COMP_U, 8>;
@@ -976,8 +605,9 @@ KFn chain_kernel(int kind, const KArgs &a) {
     }
 }
 
-KFn terms_kernel(int kind, int simd) {
-    const bool w = simd == 16;
+KFn terms_kernel(int kind, const KArgs &a) {
+    const bool w = a.simd == 16;
+    if (a.model != 1) return chain_scalar_terms(kind, a.model);
     switch (kind) {
         case PH_U: return w ? k_mom1_terms<COMP_U, 16> : k_mom1_terms<COMP_U, 8>;
         case PH_V: return w ? k_mom1_terms<COMP_V, 16> : k_mom1_terms<COMP_V, 8>;
@@ -987,7 +617,9 @@ KFn terms_kernel(int kind, int simd) {
 
 }  // namespace
 
-size_t chain_record_bytes() { return (size_t)MOM_PAIRS_MAX * KMAX_LEVELS * sizeof(float2); }
+size_t chain_record_bytes(int model) {
+    return (size_t)(model == 1 ? MOM_PAIRS_MAX : chain_scalar_pairs(model)) * KMAX_LEVELS * sizeof(float2);
+}
 
 size_t chain_unit_words(int nii, int njj) {
     return (size_t)chain_claims(nii - 2) * (njj - 2) * 2 * KMAX_LEVELS;   // two values a level at most
@@ -1023,7 +655,7 @@ void launch_chain(int kind, const KArgs &a, const SweepGeom &g, const ChainBufs 
             const int rows = std::max(1, 256 / a.ks), per = rows * PT_COLS;
             k_pressure_terms<<<dim3((a.ncols + per - 1) / per, n), dim3(a.ks, rows), 0, st>>>(a, b);
         } else {
-            terms_kernel(kind, a.simd)<<<(unsigned)tiles, CT_THREADS, 0, st>>>(a, g, b);
+            terms_kernel(kind, a)<<<(unsigned)tiles, CT_THREADS, 0, st>>>(a, g, b);
         }
         chain_kernel(kind, a)<<<grid, CH_THREADS, 0, st>>>(a, g, b);
     }

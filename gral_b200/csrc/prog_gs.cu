@@ -257,45 +257,13 @@ __device__ __forceinline__ void tke_sweep(Rows &R, const KArgs &a, const ColCtx 
         }
         R.b1(k) = PT; R.d1(k) = QT; R.b2(k) = PE; R.d2(k) = QE;
     }
-    const long long E = c.nj2, N = 1;
-    auto hyp = [](double p, double q) { return sqrt(p * p + q * q); };
     float kup = ktop, eup = etop;
     for (int k = VI; k >= K0; --k) {
         float kn = R.k1(k), en = R.e1(k);
         if (KK < k) {
-            float U;
-            bool wall = true;
-            double div;   // TDISS divisor
-            if (k == KK + 1 && (c.fl & F_CUTK0)) {
-                if (c.fl & F_GMODE1) {
-                    U = (float)(ke.gfac * hyp(0.5 * (double)(vel(0, 0, k + 1) + vel(0, E, k + 1)),
-                                              0.5 * (double)(vel(1, 0, k + 1) + vel(1, N, k + 1))));
-                    div = ((double)a.dzk[k] + (double)a.dzk[k + 1] * 0.5) * 0.4;
-                } else {
-                    U = (float)(ke.gfac * hyp(0.5 * (double)((vel(0, 0, k + 1)) + vel(0, E, k)),
-                                              0.5 * (double)((vel(1, 0, k)) + vel(1, N, k))));
-                    div = (double)a.dzk[k] * 0.5 * 0.4;
-                }
-            } else if (k == KK + 1 && (c.fl & F_CUTKGT0)) {
-                U = c.cf.help_o * (float)hyp(0.5 * (double)(vel(0, 0, k) + vel(0, E, k)),
-                                             0.5 * (double)(vel(1, 0, k) + vel(1, N, k)));
-                div = (double)a.dzk[k] * 0.5 * 0.4;
-            } else if (k == ke.kw_e || k == ke.kw_w) {
-                U = (float)((double)a.ustern_fx * hyp(0.5 * (double)(vel(2, 0, k) + vel(2, 0, k + 1)),
-                                                      0.5 * (double)(vel(1, 0, k) + vel(1, N, k))));
-                div = (double)a.building_z0 * 0.4;
-            } else if (k == ke.kw_n || k == ke.kw_s) {
-                U = (float)((double)a.ustern_fx * hyp(0.5 * (double)(vel(2, 0, k) + vel(2, 0, k + 1)),
-                                                      0.5 * (double)(vel(0, 0, k) + vel(0, E, k))));
-                div = (double)a.building_z0 * 0.4;
-            } else {
-                wall = false;
+            if (!tke_wall(a, c, ke, k, kn, en, vel)) {
                 kn = R.b1(k) * kup + R.d1(k);
                 en = R.b2(k) * eup + R.d2(k);
-            }
-            if (wall) {
-                kn = (float)(3.33 * (double)(U * U));
-                en = (float)((double)(U * U * U) / div);
             }
             kn = (float)net_maxd((double)kn, 0.001);
             en = (float)net_maxd((double)en, 0.0000001);

@@ -235,7 +235,7 @@ bool gral::fused_strips(const gral_ctx *ctx) {
     return use_strips(ctx) && ctx->pmode == 1 + strip_num_variants();
 }
 
-bool gral::use_chain(const gral_ctx *ctx) { return !ctx->il && ctx->model == 1 && ctx->pmode == kChainMode(); }
+bool gral::use_chain(const gral_ctx *ctx) { return !ctx->il && ctx->pmode == kChainMode(); }
 
 namespace {
 
@@ -251,6 +251,7 @@ void launch_iteration(gral_ctx *ctx, cudaStream_t st) {
         launch_chain(PH_U, a, ctx->geo_u.g, ctx->cb, ctx->chain_grid[PH_U], st);
         launch_chain(PH_V, a, ctx->geo_v.g, ctx->cb, ctx->chain_grid[PH_V], st);
         launch_chain(PH_W, a, ctx->geo_p.g, ctx->cb, ctx->chain_grid[PH_W], st);
+        if (ctx->model == 2) launch_chain(PH_TKE, a, ctx->geo_p.g, ctx->cb, ctx->chain_grid[PH_TKE], st);
         launch_bookkeeping(a, st);
         return;
     }
@@ -290,7 +291,7 @@ void launch_iteration(gral_ctx *ctx, cudaStream_t st) {
 int launches_per_iteration(const gral_ctx *ctx) {
     const int gs = ctx->ka.group_set <= 0 ? ctx->ngroups : ctx->ka.group_set;
     const int sets = ctx->il ? (ctx->ngroups + gs - 1) / gs : 1;
-    if (use_chain(ctx)) return 3 + 4 * 2 * ((ctx->nb + ctx->cb.unit_n - 1) / ctx->cb.unit_n) + 3;
+    if (use_chain(ctx)) return 3 + (ctx->model == 2 ? 5 : 4) * 2 * ((ctx->nb + ctx->cb.unit_n - 1) / ctx->cb.unit_n) + 3;
     if (fused_strips(ctx)) return 3 + 3 + 1;
     if (use_strips(ctx)) return 3 + 4 + 3;
     if (ctx->fused) return 3 + 1 + 2 + 1;
@@ -328,8 +329,8 @@ int size_grids(gral_ctx *ctx) {
     }
     ctx->ka.chain = use_chain(ctx) ? 1 : 0;
     if (use_chain(ctx)) {
-        const Geom *gk[4] = {&ctx->geo_p, &ctx->geo_u, &ctx->geo_v, &ctx->geo_p};
-        for (int q = 0; q < 4; ++q) {
+        const Geom *gk[5] = {&ctx->geo_p, &ctx->geo_u, &ctx->geo_v, &ctx->geo_p, &ctx->geo_p};
+        for (int q = 0; q < (ctx->model == 2 ? 5 : 4); ++q) {
             const long long claims = (long long)chain_claims(gk[q]->g.ni) * ctx->cb.unit_n;
             CK(chain_grid(kinds[q], ctx->ka, claims, &ctx->chain_grid[kinds[q]]));
         }
@@ -414,7 +415,7 @@ int tune_variants(gral_ctx *ctx) {
     return build_graph(ctx);
 }
 
-// Schedule of the slab family's model-1 sweeps.  The row chains are the fastest on every grid measured
+// Schedule of the slab family's sweeps.  The row chains are the fastest on every grid measured
 // (ms of an iteration, row chains / best other: 16x14 0.17 / 0.24, 100x100 0.60 / 1.53, 200x200 1.33 /
 // 3.54, 400x400 3.38 / 8.33), so they run wherever their buffers fit.  Otherwise the diagonal-claim
 // wavefront and the strip variants, which give bit-identical results, each run two live iterations
@@ -441,7 +442,7 @@ int tune_plain(gral_ctx *ctx) {
     const int forced_nv = kChainMode() + (ctx->chain_ok ? 1 : 0);
     const int first_stop = std::min(((ctx->it_host + ctx->cadence - 1) / ctx->cadence) * ctx->cadence, ctx->it_max);
     if (ctx->model != 1) {
-        ctx->pmode = 0;
+        ctx->pmode = ctx->chain_ok ? kChainMode() : 0;
     } else if (ctx->forced_pmode >= 0 && ctx->forced_pmode < forced_nv) {
         ctx->pmode = ctx->forced_pmode;
     } else if (ctx->chain_ok) {
@@ -516,9 +517,9 @@ constexpr size_t kChainBytes = (size_t)8 << 30;
 int reserve_chain(gral_ctx *ctx) {
     ctx->chain_ok = false;
     ctx->ka.epoch = nullptr;
-    if (ctx->il || ctx->model != 1) return GRAL_OK;
+    if (ctx->il) return GRAL_OK;
     cudaStream_t st = ctx->stream;
-    const size_t unit = chain_record_bytes() * ctx->ncols;
+    const size_t unit = chain_record_bytes(ctx->model) * ctx->ncols;
     const size_t words = chain_unit_words(ctx->nii, ctx->njj);
     int units = (int)std::max<size_t>(1, std::min<size_t>(ctx->nb, kChainBytes / unit));
     if (const char *v = std::getenv("GRAL_PROG_CHAIN_UNITS")) units = std::max(1, std::min(units, std::atoi(v)));
@@ -1139,7 +1140,9 @@ int gral_prog_iterate_timed(gral_ctx *ctx, int32_t iterations, double *phase_ms,
         seq.push_back({GRAL_PHASE_V, [&] { launch_gs(PH_V, a, ctx->geo_v.g, ctx->grid_gs[PH_V], st); }});
         seq.push_back({GRAL_PHASE_W, [&] { launch_gs(PH_W, a, ctx->geo_p.g, ctx->grid_gs[PH_W], st); }});
     }
-    if (ctx->model == 2)
+    if (ctx->model == 2 && chain)
+        seq.push_back({GRAL_PHASE_TKE, [&] { chain_phase(PH_TKE, ctx->geo_p); }});
+    else if (ctx->model == 2)
         seq.push_back({GRAL_PHASE_TKE, [&] { launch_gs(PH_TKE, a, ctx->geo_p.g, ctx->grid_gs[PH_TKE], st); }});
     seq.push_back({GRAL_PHASE_BOOKKEEPING, [&] { launch_bookkeeping(a, st); }});
     const int marks = (int)seq.size() + 1;

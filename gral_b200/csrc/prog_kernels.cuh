@@ -55,9 +55,9 @@ void launch_fused_strip(const KArgs &a, const FusedGeom &fg, int grid, cudaStrea
 cudaError_t fused_occupancy(int *blocks_per_sm);
 void launch_fused_pvau(const KArgs &a, const FusedGeom &fg, int grid, cudaStream_t st);
 
-// row-chain schedule of the slab family's model-1 sweeps: coefficient launch and chain launch of one
-// phase (kind = PH_PRESSURE, PH_U, PH_V, PH_W); bufs.unit_n situations at a time
-size_t chain_record_bytes();
+// row-chain schedule of the slab family's sweeps: coefficient launch and chain launch of one
+// phase (kind = PH_PRESSURE, PH_U, PH_V, PH_W, PH_TKE); bufs.unit_n situations at a time
+size_t chain_record_bytes(int model);
 size_t chain_unit_words(int nii, int njj);      // words of one unit
 int chain_claims(int ni);                               // claims of a sweep of ni rows
 cudaError_t chain_grid(int kind, const KArgs &a, long long claims, int *grid);

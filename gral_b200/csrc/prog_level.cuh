@@ -587,9 +587,10 @@ __device__ __forceinline__ float wind_half(float a1, float a2, float b1, float b
 }
 
 // U (COMP 0) or V (COMP 1) of models 2 (DIFF) and 0 (no DIFF), one level
-// (U-prognostic-microscale_2.cs:103-257, V-...2.cs, U-...0.cs:103-182, V-...0.cs).
+// (U-prognostic-microscale_2.cs:103-257, V-...2.cs, U-...0.cs:103-182, V-...0.cs), split like the
+// model-1 levels: everything but the swept field's four horizontal neighbours first.
 template <bool DIFF, int COMP, bool IL>
-__device__ __forceinline__ Coef uv_scalar_level(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc,
+__device__ __forceinline__ MomPre uv_scalar_pre(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc,
                                                 int k) {
     const long long W = -(long long)c.nj2, E = c.nj2, S = -1, N = 1;
     const float DXK = a.dxk, DYK = a.dyk, AREA = a.areaxy;
@@ -635,39 +636,38 @@ __device__ __forceinline__ Coef uv_scalar_level(const KArgs &a, const Acc<IL> &x
         FT = 0.25f * (wksS + wks + a.wks[x.at(S, k + 1)] + a.wks[x.at(0, k + 1)]) * AREA;
         if (k > c.KK + 1) FB = 0.25f * (wksS + wks + a.wks[x.at(S, k - 1)] + a.wks[x.at(0, k - 1)]) * AREA;
     }
-    Coef r;
-    float AE1, AW1, AS1, AN1;
+    MomPre r;
     if (DIFF) {
         DE = vmaxf(DE, 0.0001f); DB = vmaxf(DB, 0.0001f); DW = vmaxf(DW, 0.0001f);
         DS = vmaxf(DS, 0.0001f); DN = vmaxf(DN, 0.0001f); DT = vmaxf(DT, 0.0001f);
         r.B = pl_ke(DT, fabsf(FT / DT), -FT);
         r.C = pl_ke(DB, fabsf(FB / DB), FB);
-        AE1 = pl_ke(DE, fabsf(FE / DE), -FE);
-        AW1 = pl_ke(DW, fabsf(FW / DW), FW);
-        AS1 = pl_ke(DS, fabsf(FS / DS), FS);
-        AN1 = pl_ke(DN, fabsf(FN / DN), -FN);
+        r.ae = pl_ke(DE, fabsf(FE / DE), -FE);
+        r.aw = pl_ke(DW, fabsf(FW / DW), FW);
+        r.as = pl_ke(DS, fabsf(FS / DS), FS);
+        r.an = pl_ke(DN, fabsf(FN / DN), -FN);
     } else {                                                  // upwind, U-prognostic-microscale_0.cs:123-128
         r.B = vmaxf(-FT, 0.0f);
         r.C = vmaxf(FB, 0.0f);
-        AE1 = vmaxf(-FE, 0.0f);
-        AW1 = vmaxf(FW, 0.0f);
-        AS1 = vmaxf(FS, 0.0f);
-        AN1 = vmaxf(-FN, 0.0f);
+        r.ae = vmaxf(-FE, 0.0f);
+        r.aw = vmaxf(FW, 0.0f);
+        r.as = vmaxf(FS, 0.0f);
+        r.an = vmaxf(-FN, 0.0f);
     }
     const float ap0 = sc.ap0[k];
-    r.A = r.B + r.C + AW1 + AS1 + AE1 + AN1 + ap0;
-    const float pW = __ldcg(PHI + x.at(W, k)), pE = __ldcg(PHI + x.at(E, k));
-    const float pS = __ldcg(PHI + x.at(S, k)), pN = __ldcg(PHI + x.at(N, k));
-    float DIM;
+    r.A = r.B + r.C + r.aw + r.as + r.ae + r.an + ap0;
     if (COMP == 0) {
         const float DDPX = a.dpmnew[x.at(W, k)] - a.dpmnew[x.at(0, k)];
-        DIM = (float)(AW1 * pW + AS1 * pS + AE1 * pE + AN1 * pN + ap0 * 0.5 * (uksW + uks) + DDPX * dydz +
-                      a.coriolis * (sc.ug - phi) * AREA * dz);
+        r.t1 = uksW + uks;
+        r.t2 = DDPX * dydz;
+        r.t3 = a.coriolis * (sc.ug - phi) * AREA * dz;
     } else {
         const float DDPY = a.dpmnew[x.at(S, k)] - a.dpmnew[x.at(0, k)];
-        DIM = (float)(AW1 * pW + AS1 * pS + AE1 * pE + AN1 * pN + ap0 * 0.5 * (a.vks[x.at(S, k)] + vks) + DDPY * dxdz +
-                      a.coriolis * (sc.vg - phi) * AREA * dz);
+        r.t1 = a.vks[x.at(S, k)] + vks;
+        r.t2 = DDPY * dxdz;
+        r.t3 = a.coriolis * (sc.vg - phi) * AREA * dz;
     }
+    r.w = 0.0f;
     if (k == c.KK + 1) {                                      // wall law, U-prognostic-microscale_2.cs:205-231
         const float windhilf = vmaxf(wind_half(uksW, uks, vksW, vks), 0.01f);
         float Ust;
@@ -679,41 +679,62 @@ __device__ __forceinline__ Coef uv_scalar_level(const KArgs &a, const Acc<IL> &x
         } else {
             Ust = c.cf.help_o * windhilf;
         }
-        DIM -= (float)(phi / windhilf * (Ust * Ust) * AREA);
+        r.w = (float)(phi / windhilf * (Ust * Ust) * AREA);
     }
-    if (DIFF && k > c.KK + 1) {                               // :234-245
-        float ADD;
+    r.vdx = r.e0 = r.e1 = r.e2 = r.e3 = 0.0f;
+    r.hz = (COMP == 0) ? dydz : dxdz;
+    if (DIFF && k > c.KK + 1) {                               // :234-245, the pieces without the swept field
+        r.vdx = VIS / DXK;
+        const float wksB = a.wks[x.at(0, k - 1)];
         if (COMP == 0) {
-            const float DUDXE = (pE - phi) * dydz;
-            const float DUDXW = (phi - pW) * dydz;
-            const float vksN = a.vks[x.at(N, k)], vksS = a.vks[x.at(S, k)];
-            const float DVDXN = (0.5f * (a.vks[x.at(E + N, k)] + vksN) - 0.5f * (vksN + a.vks[x.at(W + N, k)])) * dxdz;
-            const float DVDXS = (0.5f * (a.vks[x.at(E + S, k)] + vksS) - 0.5f * (vksS + a.vks[x.at(W + S, k)])) * dxdz;
-            const float wksW = a.wks[x.at(W, k)], wksB = a.wks[x.at(0, k - 1)];
-            const float DWDXT = (0.5f * (a.wk[x.at(E, k)] + wks) - 0.5f * (wks + wksW)) * AREA;
-            const float DWDXB = (0.5f * (a.wk[x.at(E, k - 1)] + wksB) - 0.5f * (wksB + a.wks[x.at(W, k - 1)])) * AREA;
-            ADD = VIS / DXK * (DUDXE - DUDXW + DVDXN - DVDXS + DWDXT - DWDXB);
+            const float vksN = a.vks[x.at(N, k)], vksS = a.vks[x.at(S, k)], wksW = a.wks[x.at(W, k)];
+            r.e0 = (0.5f * (a.vks[x.at(E + N, k)] + vksN) - 0.5f * (vksN + a.vks[x.at(W + N, k)])) * dxdz;   // DVDXN
+            r.e1 = (0.5f * (a.vks[x.at(E + S, k)] + vksS) - 0.5f * (vksS + a.vks[x.at(W + S, k)])) * dxdz;   // DVDXS
+            r.e2 = (0.5f * (a.wk[x.at(E, k)] + wks) - 0.5f * (wks + wksW)) * AREA;                           // DWDXT
+            r.e3 = (0.5f * (a.wk[x.at(E, k - 1)] + wksB) - 0.5f * (wksB + a.wks[x.at(W, k - 1)])) * AREA;    // DWDXB
         } else {
-            const float DVDYN = (pN - phi) * dxdz;
-            const float DVDYS = (phi - pS) * dxdz;
-            const float uksE = a.uks[x.at(E, k)];
+            const float uksE = a.uks[x.at(E, k)], wksS = a.wks[x.at(S, k)];
             const float DUDYE = (0.5f * (a.uks[x.at(E + N, k)] + uksE) - 0.5f * (uksE + a.uks[x.at(E + S, k)])) * dxdz;
             const float DUDYW = (0.5f * (a.uks[x.at(W + N, k)] + uksW) - 0.5f * (uksW + a.uks[x.at(W + S, k)])) * dxdz;
-            const float wksS = a.wks[x.at(S, k)], wksB = a.wks[x.at(0, k - 1)];
-            const float DWDYT = (0.5f * (a.wk[x.at(N, k)] + wks) - 0.5f * (wks + wksS)) * AREA;
-            const float DWDYB = (0.5f * (a.wk[x.at(N, k - 1)] + wksB) - 0.5f * (wksB + a.wks[x.at(S, k - 1)])) * AREA;
-            ADD = VIS / DXK * (DUDYE - DUDYW + DVDYN - DVDYS + DWDYT - DWDYB);
+            r.e0 = DUDYE - DUDYW;
+            r.e1 = (0.5f * (a.wk[x.at(N, k)] + wks) - 0.5f * (wks + wksS)) * AREA;                           // DWDYT
+            r.e2 = (0.5f * (a.wk[x.at(N, k - 1)] + wksB) - 0.5f * (wksB + a.wks[x.at(S, k - 1)])) * AREA;    // DWDYB
         }
-        DIM += ADD;
     }
-    r.D = DIM;
     r.phi = phi;
     return r;
 }
 
+// DIM of one level: the source sum is partly in double, then the wall law and the viscous terms
+template <bool DIFF, int COMP>
+__device__ __forceinline__ float uv_scalar_post(const MomPre &p, const ColCtx &c, int k, float ap0, float nW, float nS,
+                                                float nE, float nN) {
+    float DIM = (float)(p.aw * nW + p.as * nS + p.ae * nE + p.an * nN + ap0 * 0.5 * p.t1 + p.t2 + p.t3);
+    if (k == c.KK + 1) DIM -= p.w;
+    if (DIFF && k > c.KK + 1) {
+        if (COMP == 0) {
+            const float DUDXE = (nE - p.phi) * p.hz, DUDXW = (p.phi - nW) * p.hz;
+            DIM += p.vdx * (DUDXE - DUDXW + p.e0 - p.e1 + p.e2 - p.e3);
+        } else {
+            const float DVDYN = (nN - p.phi) * p.hz, DVDYS = (p.phi - nS) * p.hz;
+            DIM += p.vdx * (p.e0 + DVDYN - DVDYS + p.e1 - p.e2);
+        }
+    }
+    return DIM;
+}
+
+template <bool DIFF, int COMP, bool IL>
+__device__ __forceinline__ Coef uv_scalar_level(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc,
+                                                int k) {
+    const MomPre p = uv_scalar_pre<DIFF, COMP, IL>(a, x, c, sc, k);
+    float nW, nS, nE, nN;
+    nbr4(COMP == 0 ? a.uk : a.vk, x, c, k, nW, nS, nE, nN);
+    return Coef{p.A, p.B, p.C, uv_scalar_post<DIFF, COMP>(p, c, k, sc.ap0[k], nW, nS, nE, nN), p.phi};
+}
+
 // W of models 2 (DIFF) and 0, one level (W-prognostic-microscale_2.cs:84-199, W-...0.cs:84-123).
 template <bool DIFF, bool IL>
-__device__ __forceinline__ Coef w_scalar_level(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc,
+__device__ __forceinline__ MomPre w_scalar_pre(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc,
                                                int k) {
     const long long W = -(long long)c.nj2, E = c.nj2, S = -1, N = 1;
     const float DXK = a.dxk, DYK = a.dyk, AREA = a.areaxy;
@@ -745,31 +766,30 @@ __device__ __forceinline__ Coef w_scalar_level(const KArgs &a, const Acc<IL> &x,
     const float wks = a.wks[x.at(0, k)], wksB = a.wks[x.at(0, k - 1)];
     const float FT = wks * AREA;
     const float FB = (k > c.KK + 1) ? wksB * AREA : 0.0f;
-    Coef r;
-    float AE1, AW1, AS1, AN1;
+    MomPre r;
     if (DIFF) {
         DE = vmaxf(DE, 0.0001f); DB = vmaxf(DB, 0.0001f); DW = vmaxf(DW, 0.0001f);
         DS = vmaxf(DS, 0.0001f); DN = vmaxf(DN, 0.0001f); DT = vmaxf(DT, 0.0001f);
         r.B = pl_ke(DT, fabsf(FT / DT), -FT);
         r.C = pl_ke(DB, fabsf(FB / DB), FB);
-        AE1 = pl_ke(DE, fabsf(FE / DE), -FE);
-        AW1 = pl_ke(DW, fabsf(FW / DW), FW);
-        AS1 = pl_ke(DS, fabsf(FS / DS), FS);
-        AN1 = pl_ke(DN, fabsf(FN / DN), -FN);
+        r.ae = pl_ke(DE, fabsf(FE / DE), -FE);
+        r.aw = pl_ke(DW, fabsf(FW / DW), FW);
+        r.as = pl_ke(DS, fabsf(FS / DS), FS);
+        r.an = pl_ke(DN, fabsf(FN / DN), -FN);
     } else {
         r.B = vmaxf(-FT, 0.0f);
         r.C = vmaxf(FB, 0.0f);
-        AE1 = vmaxf(-FE, 0.0f);
-        AW1 = vmaxf(FW, 0.0f);
-        AS1 = vmaxf(FS, 0.0f);
-        AN1 = vmaxf(-FN, 0.0f);
+        r.ae = vmaxf(-FE, 0.0f);
+        r.aw = vmaxf(FW, 0.0f);
+        r.as = vmaxf(FS, 0.0f);
+        r.an = vmaxf(-FN, 0.0f);
     }
     const float ap0 = sc.ap0[k];
-    r.A = r.B + r.C + AW1 + AS1 + AE1 + AN1 + ap0;
+    r.A = r.B + r.C + r.aw + r.as + r.ae + r.an + ap0;
     const float DDPZ = a.dpmnew[x.at(0, k - 1)] - a.dpmnew[x.at(0, k)];
-    const float wW = __ldcg(a.wk + x.at(W, k)), wS = __ldcg(a.wk + x.at(S, k));
-    const float wE = __ldcg(a.wk + x.at(E, k)), wN = __ldcg(a.wk + x.at(N, k));
-    float DIM = (float)(AW1 * wW + AS1 * wS + AE1 * wE + AN1 * wN + ap0 * 0.5 * (wksB + wks) + DDPZ * AREA);
+    r.t1 = wksB + wks;
+    r.t2 = DDPZ * AREA;
+    r.e0 = 0.0f;
     if (DIFF && k > c.KK + 1) {                               // W-prognostic-microscale_2.cs:162-172
         const float DUDZE = (0.5f * (a.uks[x.at(0, k + 1)] + uks) - 0.5f * (uks + uksM)) * dydz;
         const float DUDZW = (0.5f * (a.uks[x.at(W, k + 1)] + uksW) - 0.5f * (uksW + a.uks[x.at(W, k - 1)])) * dydz;
@@ -777,11 +797,27 @@ __device__ __forceinline__ Coef w_scalar_level(const KArgs &a, const Acc<IL> &x,
         const float DVDZS = (0.5f * (a.vks[x.at(S, k + 1)] + vksS) - 0.5f * (vksS + a.vks[x.at(S, k - 1)])) * dxdz;
         const float DWDZT = (__ldcg(a.wk + x.at(0, k + 1)) - wk) * AREA;
         const float DWDZB = (wk - __ldcg(a.wk + x.at(0, k - 1))) * AREA;
-        DIM += VIS / dz * (DUDZE - DUDZW + DVDZN - DVDZS + DWDZT - DWDZB);
+        r.e0 = VIS / dz * (DUDZE - DUDZW + DVDZN - DVDZS + DWDZT - DWDZB);
     }
-    r.D = DIM;
     r.phi = wk;
     return r;
+}
+
+template <bool DIFF>
+__device__ __forceinline__ float w_scalar_post(const MomPre &p, const ColCtx &c, int k, float ap0, float nW, float nS,
+                                               float nE, float nN) {
+    float DIM = (float)(p.aw * nW + p.as * nS + p.ae * nE + p.an * nN + ap0 * 0.5 * p.t1 + p.t2);
+    if (DIFF && k > c.KK + 1) DIM += p.e0;
+    return DIM;
+}
+
+template <bool DIFF, bool IL>
+__device__ __forceinline__ Coef w_scalar_level(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc,
+                                               int k) {
+    const MomPre p = w_scalar_pre<DIFF, IL>(a, x, c, sc, k);
+    float nW, nS, nE, nN;
+    nbr4(a.wk, x, c, k, nW, nS, nE, nN);
+    return Coef{p.A, p.B, p.C, w_scalar_post<DIFF>(p, c, k, sc.ap0[k], nW, nS, nE, nN), p.phi};
 }
 
 // Coefficients of the turbulent kinetic energy k and its dissipation eps at one level
@@ -790,9 +826,14 @@ struct CoefKE {
     float A, B1, C1, D1, B2, C2, D2, k1, e1;
 };
 
+// ... without the four horizontal neighbours of TURB and TDISS: neighbour coefficients and, in the
+// reference's order, the source terms that follow the neighbour products
+struct KePre {
+    float A, B1, C1, B2, C2, aw, as, ae, an, t1, t2, t3, s1, s2, k1, e1;
+};
+
 template <bool IL>
-__device__ __forceinline__ CoefKE tke_level(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc,
-                                            int k) {
+__device__ __forceinline__ KePre tke_pre(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc, int k) {
     const float potdtdz = sc.potdtdz;
     const long long W = -(long long)c.nj2, E = c.nj2, S = -1, N = 1;
     const float DXK = a.dxk, DYK = a.dyk, AREA = a.areaxy;
@@ -835,17 +876,17 @@ __device__ __forceinline__ CoefKE tke_level(const KArgs &a, const Acc<IL> &x, co
     const float PBEPS = fabsf(FN / DBEPS);                      // FN, not FB (:187)
     const float PTEPS = fabsf(FT / DTEPS);
     auto p5 = [](float v) { const float q = 1 - 0.1f * v; return q * q * q * q * q; };
-    CoefKE r;
+    KePre r;
     r.B1 = DT * net_maxf(0, p5(PT)) + net_maxf(-FT, 0);
     r.C1 = DB * net_maxf(0, p5(PB)) + net_maxf(FB, 0);
-    const float AE1 = DE * net_maxf(0, p5(PE)) + net_maxf(-FE, 0);
-    const float AW1 = DW * net_maxf(0, p5(PW)) + net_maxf(FW, 0);
-    const float AS1 = DS * net_maxf(0, p5(PS)) + net_maxf(FS, 0);
-    const float AN1 = DN * net_maxf(0, p5(PN)) + net_maxf(-FN, 0);
+    r.ae = DE * net_maxf(0, p5(PE)) + net_maxf(-FE, 0);
+    r.aw = DW * net_maxf(0, p5(PW)) + net_maxf(FW, 0);
+    r.as = DS * net_maxf(0, p5(PS)) + net_maxf(FS, 0);
+    r.an = DN * net_maxf(0, p5(PN)) + net_maxf(-FN, 0);
     r.B2 = DT * net_maxf(0, p5(PTEPS)) + net_maxf(-FT, 0);
     r.C2 = DB * net_maxf(0, p5(PBEPS)) + net_maxf(FB, 0);
     const float ap0 = sc.ap0[k];
-    r.A = r.B1 + r.C1 + AW1 + AS1 + AE1 + AN1 + ap0;
+    r.A = r.B1 + r.C1 + r.aw + r.as + r.ae + r.an + ap0;
     // production terms (:213-243)
     const float UX1 = UKip, UX2 = UK;
     const float VX1 = 0.5f * (a.vk[x.at(E, k)] + a.vk[x.at(E + N, k)]);
@@ -875,15 +916,71 @@ __device__ __forceinline__ CoefKE tke_level(const KArgs &a, const Acc<IL> &x, co
     const float PROTURB = VIS * AREA * dz *
         (2 * sq(DUDX) + 2 * sq(DVDY) + 2 * sq(DWDZ) + sq(DUDY + DVDX) + sq(DUDZ + DWDX) + sq(DVDZ + DWDY) - TDISS);
     const float PROBOU = (float)(-potdtdz * 9.81 / 283 * VIS * 1.35 * AREA * dz);
-    const float tW = __ldcg(a.turb + x.at(W, k)), tS = __ldcg(a.turb + x.at(S, k));
-    const float tE = __ldcg(a.turb + x.at(E, k)), tN = __ldcg(a.turb + x.at(N, k));
-    const float eW = __ldcg(a.tdiss + x.at(W, k)), eS = __ldcg(a.tdiss + x.at(S, k));
-    const float eE = __ldcg(a.tdiss + x.at(E, k)), eN = __ldcg(a.tdiss + x.at(N, k));
-    r.D1 = AW1 * tW + AS1 * tS + AE1 * tE + AN1 * tN + ap0 * TURB + PROTURB + PROBOU;
-    r.D2 = AW1 * eW + AS1 * eS + AE1 * eE + AN1 * eN + ap0 * TDISS + (TDISS / TURB * (1.44f * PROTURB - 1.92f * TDISS));
+    r.t1 = ap0 * TURB;
+    r.t2 = PROTURB;
+    r.t3 = PROBOU;
+    r.s1 = ap0 * TDISS;
+    r.s2 = TDISS / TURB * (1.44f * PROTURB - 1.92f * TDISS);
     r.k1 = TURB;
     r.e1 = TDISS;
     return r;
+}
+
+template <bool IL>
+__device__ __forceinline__ CoefKE tke_level(const KArgs &a, const Acc<IL> &x, const ColCtx &c, const SitCtx &sc,
+                                            int k) {
+    const KePre p = tke_pre<IL>(a, x, c, sc, k);
+    float tW, tS, tE, tN, eW, eS, eE, eN;
+    nbr4(a.turb, x, c, k, tW, tS, tE, tN);
+    nbr4(a.tdiss, x, c, k, eW, eS, eE, eN);
+    CoefKE r;
+    r.A = p.A; r.B1 = p.B1; r.C1 = p.C1; r.B2 = p.B2; r.C2 = p.C2;
+    r.D1 = p.aw * tW + p.as * tS + p.ae * tE + p.an * tN + p.t1 + p.t2 + p.t3;
+    r.D2 = p.aw * eW + p.as * eS + p.ae * eE + p.an * eN + p.s1 + p.s2;
+    r.k1 = p.k1;
+    r.e1 = p.e1;
+    return r;
+}
+
+// Wall functions of the k-eps back-substitution at a level above KKART: ground, roof and the four
+// neighbour walls (TKE-prognostic-microscale.cs:272-343).  False where the level is solved instead.
+// vel(field, dc, k) loads UK/VK/WK of the column (dc = 0) or its east/north neighbour.
+template <class Vel>
+__device__ __forceinline__ bool tke_wall(const KArgs &a, const ColCtx &c, const ColKE &ke, int k, float &kn, float &en,
+                                         Vel &&vel) {
+    const long long E = c.nj2, N = 1;
+    const int KK = c.KK;
+    auto hyp = [](double p, double q) { return sqrt(p * p + q * q); };
+    float U;
+    double div;   // TDISS divisor
+    if (k == KK + 1 && (c.fl & F_CUTK0)) {
+        if (c.fl & F_GMODE1) {
+            U = (float)(ke.gfac * hyp(0.5 * (double)(vel(0, 0, k + 1) + vel(0, E, k + 1)),
+                                      0.5 * (double)(vel(1, 0, k + 1) + vel(1, N, k + 1))));
+            div = ((double)a.dzk[k] + (double)a.dzk[k + 1] * 0.5) * 0.4;
+        } else {
+            U = (float)(ke.gfac * hyp(0.5 * (double)((vel(0, 0, k + 1)) + vel(0, E, k)),
+                                      0.5 * (double)((vel(1, 0, k)) + vel(1, N, k))));
+            div = (double)a.dzk[k] * 0.5 * 0.4;
+        }
+    } else if (k == KK + 1 && (c.fl & F_CUTKGT0)) {
+        U = c.cf.help_o * (float)hyp(0.5 * (double)(vel(0, 0, k) + vel(0, E, k)),
+                                     0.5 * (double)(vel(1, 0, k) + vel(1, N, k)));
+        div = (double)a.dzk[k] * 0.5 * 0.4;
+    } else if (k == ke.kw_e || k == ke.kw_w) {
+        U = (float)((double)a.ustern_fx * hyp(0.5 * (double)(vel(2, 0, k) + vel(2, 0, k + 1)),
+                                              0.5 * (double)(vel(1, 0, k) + vel(1, N, k))));
+        div = (double)a.building_z0 * 0.4;
+    } else if (k == ke.kw_n || k == ke.kw_s) {
+        U = (float)((double)a.ustern_fx * hyp(0.5 * (double)(vel(2, 0, k) + vel(2, 0, k + 1)),
+                                              0.5 * (double)(vel(0, 0, k) + vel(0, E, k))));
+        div = (double)a.building_z0 * 0.4;
+    } else {
+        return false;
+    }
+    kn = (float)(3.33 * (double)(U * U));
+    en = (float)((double)(U * U * U) / div);
+    return true;
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1,4 +1,4 @@
-"""The row-chain schedule (the slab family's default for model 1) against the oracle, bit for bit.
+"""The row-chain schedule (the slab family's default) against the oracle, bit for bit.
 
 Its claims are 32 sweep rows (8 blocks of 4), so the grids put the sweeps' row counts (NII-2 and
 NII-3) below, at and above a block's and a claim's rows and over several claims; odd row lengths;
@@ -30,24 +30,30 @@ def domain(nii, njj, dx, dy, hills):
     return prep.make_domain(nii, njj, dx, 2.0, 1.05, 18, bl, dyk=dy)
 
 
-@pytest.mark.parametrize("nii,njj,dx,dy,simd,n,units,hills", [
-    (6, 5, 2.0, 2.0, 8, 1, 0, False),        # 4 and 3 rows: one block, not full for U
-    (7, 40, 2.5, 2.5, 8, 1, 0, False),       # 5 and 4 rows
-    (34, 9, 2.0, 4.0, 16, 1, 0, False),      # 32 and 31 rows: one claim, full and not
-    (35, 33, 3.0, 2.0, 8, 1, 0, True),       # 33 and 32 rows: a second claim of one row
-    (67, 21, 2.0, 2.0, 16, 1, 0, True),      # 65 and 64 rows: three claims and two
-    (41, 30, 2.0, 2.0, 8, 3, 0, True),       # three situations in one launch
-    (41, 30, 2.0, 2.5, 8, 3, 2, False),      # ... in sets of two
+@pytest.mark.parametrize("nii,njj,dx,dy,simd,n,units,hills,model", [
+    (6, 5, 2.0, 2.0, 8, 1, 0, False, 1),        # 4 and 3 rows: one block, not full for U
+    (7, 40, 2.5, 2.5, 8, 1, 0, False, 1),       # 5 and 4 rows
+    (34, 9, 2.0, 4.0, 16, 1, 0, False, 1),      # 32 and 31 rows: one claim, full and not
+    (35, 33, 3.0, 2.0, 8, 1, 0, True, 1),       # 33 and 32 rows: a second claim of one row
+    (67, 21, 2.0, 2.0, 16, 1, 0, True, 1),      # 65 and 64 rows: three claims and two
+    (41, 30, 2.0, 2.0, 8, 3, 0, True, 1),       # three situations in one launch
+    (6, 5, 2.0, 2.0, 8, 1, 0, False, 0),     # models 0 and 2 at the same edges
+    (34, 9, 2.5, 4.0, 8, 1, 0, False, 2),
+    (35, 33, 2.0, 2.0, 8, 1, 0, True, 2),
+    (67, 21, 3.0, 2.0, 8, 1, 0, True, 0),
+    (41, 30, 2.0, 2.0, 8, 3, 2, False, 0),
+    (41, 30, 2.0, 2.5, 8, 3, 2, True, 2),
+    (41, 30, 2.0, 2.5, 8, 3, 2, False, 1),      # ... in sets of two
 ])
-def test_chain_matches_oracle(gpu_required, monkeypatch, nii, njj, dx, dy, simd, n, units, hills):
+def test_chain_matches_oracle(gpu_required, monkeypatch, nii, njj, dx, dy, simd, n, units, hills, model):
     dom = domain(nii, njj, dx, dy, hills)
     monkeypatch.setenv("GRAL_PROG_LAYOUT", "slab")
     monkeypatch.setenv("GRAL_PROG_PLAIN_MODE", "6")
     if units:
         monkeypatch.setenv("GRAL_PROG_CHAIN_UNITS", str(units))
     sits = [prep.random_situation(900 + nii + q) for q in range(n)]
-    ps = [dom.params(x, model=1, iterations=ITERS, simd_width=simd) for x in sits]
-    f0 = [prep.initial_fields(dom, x, 1) for x in sits]
+    ps = [dom.params(x, model=model, iterations=ITERS, simd_width=simd) for x in sits]
+    f0 = [prep.initial_fields(dom, x, model) for x in sits]
     fg = [f.copy() for f in f0]
     tg = [np.zeros(ITERS, np.float32) for _ in range(n)]
     with PrognosticSolver(dom.nii, dom.njj, dom.nkk, dom.kadvmax, max_batch=n) as s:
@@ -57,6 +63,6 @@ def test_chain_matches_oracle(gpu_required, monkeypatch, nii, njj, dx, dy, simd,
         fc = f0[b].copy()
         tc = np.zeros(ITERS, np.float32)
         O.solve(ps[b], dom.static, fc, tc)
-        for name in ("uk", "vk", "wk"):
+        for name in ("uk", "vk", "wk") + (("turb", "tdiss") if model == 2 else ()):
             np.testing.assert_array_equal(getattr(fg[b], name), getattr(fc, name), err_msg=(b, name))
         np.testing.assert_array_equal(tg[b], tc)
