@@ -555,7 +555,7 @@ struct PressChain {
 
 // The kernels take the sweep's direction from the iteration count and run the code built for it.
 template <int COMP, int SW>
-__global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 1) k_mom_chain(KArgs a, SweepGeom g, ChainBufs b) {
+__global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 2) k_mom_chain(KArgs a, SweepGeom g, ChainBufs b) {
     __shared__ ChainSmem<CH_SR, 1> sm;
     constexpr int PH = COMP == COMP_U ? PH_U : (COMP == COMP_V ? PH_V : PH_W);
     constexpr int SR = CH_SR, M = CH_M, CL = CH_CL;
@@ -573,7 +573,7 @@ __global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 1) k
 }
 
 template <bool P2>
-__global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 1) k_pressure_chain(KArgs a, SweepGeom g, ChainBufs b) {
+__global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 2) k_pressure_chain(KArgs a, SweepGeom g, ChainBufs b) {
     __shared__ ChainSmem<CH_SR, 2> sm;
     constexpr int PH = PH_PRESSURE, SR = CH_SR, M = CH_M, CL = CH_CL;
     for (unsigned q = threadIdx.x; q < sizeof(sm.ring) / 8; q += CH_THREADS) sm.ring[q] = 0ull;

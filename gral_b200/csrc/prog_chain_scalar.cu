@@ -733,7 +733,7 @@ struct JobOf<2, PH_TKE, IS, JS> {
 };
 
 template <int MODEL, int KIND>
-__global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 1) k_scal_chain(KArgs a, SweepGeom g, ChainBufs b) {
+__global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 2) k_scal_chain(KArgs a, SweepGeom g, ChainBufs b) {
     __shared__ ChainSmem<CH_SR, JobOf<MODEL, KIND, 1, 1>::T::NV> sm;
     constexpr int SR = CH_SR, M = CH_M, CL = CH_CL;
     for (unsigned q = threadIdx.x; q < sizeof(sm.ring) / 8; q += CH_THREADS) sm.ring[q] = 0ull;

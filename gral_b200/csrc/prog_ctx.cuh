@@ -66,7 +66,7 @@ struct gral_ctx {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[4] = {};
     int cap_nii = 0, cap_njj = 0, cap_nkk = 0, cap_kadv = 0, cap_batch = 0;
-    int il_min_batch = 32;
+    int il_min_batch = 0;      // GRAL_PROG_LAYOUT: smallest interleaved batch (0: by interleaved_pays)
     int forced_variant = -1;   // GRAL_PROG_BATCH_VARIANT
     int lookahead = 8;         // GRAL_PROG_LOOKAHEAD: plain-family warps per average diagonal width
     int lookahead_p = 3;       // GRAL_PROG_LOOKAHEAD_P: the same for the pressure sweep

@@ -177,6 +177,18 @@ Geom make_geom(int ia, int ni, int ja, int nj) {
     return G;
 }
 
+// Whether a batch runs faster in the interleaved layout.  A batched sweep waits for its wavefront (a per
+// diagonal) and works through its groups of 32 (b per column and group); the row chains take p per
+// column and situation.  ms of an iteration, fitted to 100x100 .. 400x400 grids with 32 to 144
+// situations; measured row chains / interleaved, model 1: 48 of 100x100 3.9 / 8.4, 64 of 200x200 20.7 /
+// 20.3; model 2: 64 of 100x100 11.0 / 14.2, of 200x200 42.8 / 38.9; model 0: 6.9 / 8.6 and 25.7 / 22.9.
+bool interleaved_pays(int n, int nii, int njj, int model) {
+    if (n < 32) return false;
+    static const double P[3] = {9.9e-6, 7.9e-6, 16.4e-6}, A[3] = {0.042, 0.033, 0.072}, B[3] = {0.049e-3, 0.094e-3, 0.074e-3};
+    const double cols = (double)nii * njj, groups = (n + 31) / 32;
+    return P[model] * n * cols > A[model] * (nii + njj) + B[model] * groups * cols;
+}
+
 int validate(gral_ctx *ctx, int n, const gral_params *p, const gral_static *s, const gral_fields *f) {
     if (!ctx) return GRAL_EINVAL;
     if (n < 1 || n > ctx->cap_batch) return fail(ctx, GRAL_EINVAL, "batch size outside 1..max_batch");
@@ -512,7 +524,7 @@ int run_diagnostic(gral_ctx *ctx) {
 // situations are independent, so sets of them run one after the other), the words between strips and
 // the elimination table of the pressure sweep, built here.  If they do not fit on the device the
 // strip schedule, which needs none of them, stays the default.
-constexpr size_t kChainBytes = (size_t)8 << 30;
+constexpr size_t kChainBytes = (size_t)16 << 30;
 
 int reserve_chain(gral_ctx *ctx) {
     ctx->chain_ok = false;
@@ -524,10 +536,17 @@ int reserve_chain(gral_ctx *ctx) {
     int units = (int)std::max<size_t>(1, std::min<size_t>(ctx->nb, kChainBytes / unit));
     if (const char *v = std::getenv("GRAL_PROG_CHAIN_UNITS")) units = std::max(1, std::min(units, std::atoi(v)));
     units = std::max(units, (ctx->nb + kCounterSlots - 1) / kCounterSlots);
+    const int sets = (ctx->nb + units - 1) / units;
+    units = (ctx->nb + sets - 1) / sets;              // sets of equal size
     const size_t had = ctx->cwords.n;
     const int had_int = (int)ctx->cint.n;
     constexpr int kPasses = 8;     // flags of the table's passes, reused round by round
     cudaError_t e = ctx->crec.ensure(unit / sizeof(float2) * units);
+    while (e == cudaErrorMemoryAllocation && units > std::max(1, (ctx->nb + kCounterSlots - 1) / kCounterSlots)) {
+        cudaGetLastError();
+        units = (units + 1) / 2;
+        e = ctx->crec.ensure(unit / sizeof(float2) * units);
+    }
     if (e == cudaSuccess) e = ctx->cwords.ensure(words * ctx->nb);
     if (e == cudaSuccess) e = ctx->cptab.ensure((size_t)2 * ctx->ncols * ctx->ks);
     if (e == cudaSuccess) e = ctx->cint.ensure(1 + kPasses);
@@ -609,9 +628,9 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
     const int NII = p0.nii, NJJ = p0.njj, NKK = p0.nkk, nj2 = NJJ + 2, ncols = (NII + 2) * nj2;
     const int nk2 = NKK + 2;
     const int ks = ((p0.kadvmax + 2) + 7) / 8 * 8;
-    // Layout: batches of at least il_min_batch situations use the interleaved layout and the
-    // lane-per-situation kernels; smaller ones the slab layout and the warp-per-column kernels.
-    const bool il = n >= ctx->il_min_batch;
+    // Layout: batches for which it is the faster one use the interleaved layout and the
+    // lane-per-situation kernels, the others the slab layout and the row chains.
+    const bool il = ctx->il_min_batch > 0 ? n >= ctx->il_min_batch : interleaved_pays(n, NII, NJJ, p0.turbulence_model);
     const int ngroups = (n + 31) / 32;
     ctx->il = il;
     ctx->ngroups = ngroups;

@@ -66,3 +66,28 @@ def test_chain_matches_oracle(gpu_required, monkeypatch, nii, njj, dx, dy, simd,
         for name in ("uk", "vk", "wk") + (("turb", "tdiss") if model == 2 else ()):
             np.testing.assert_array_equal(getattr(fg[b], name), getattr(fc, name), err_msg=(b, name))
         np.testing.assert_array_equal(tg[b], tc)
+
+
+@pytest.mark.parametrize("model", [0, 1, 2])
+def test_batch_on_row_chains_equals_interleaved(gpu_required, monkeypatch, model):
+    """A batch above 32 situations on a small grid takes the row chains by itself; forced into the
+    interleaved layout it gives the same fields and traces."""
+    dom = domain(23, 19, 2.0, 2.0, False)
+    n = 33
+    sits = [prep.random_situation(700 + q) for q in range(n)]
+    ps = [dom.params(x, model=model, iterations=ITERS) for x in sits]
+    f0 = [prep.initial_fields(dom, x, model) for x in sits]
+    res = []
+    for lay in (None, "interleaved"):
+        if lay:
+            monkeypatch.setenv("GRAL_PROG_LAYOUT", lay)
+        f = [x.copy() for x in f0]
+        tr = [np.zeros(ITERS, np.float32) for _ in range(n)]
+        with PrognosticSolver(dom.nii, dom.njj, dom.nkk, dom.kadvmax, max_batch=n) as s:
+            st = s.calculate_batch(ps, dom.static, f, tr)
+        assert st[0]["layout"] == (1 if lay else 0)
+        res.append((f, tr))
+    for b in range(n):
+        for name in ("uk", "vk", "wk") + (("turb", "tdiss") if model == 2 else ()):
+            np.testing.assert_array_equal(getattr(res[0][0][b], name), getattr(res[1][0][b], name), err_msg=(b, name))
+        np.testing.assert_array_equal(res[0][1][b], res[1][1][b])
