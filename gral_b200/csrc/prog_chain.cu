@@ -589,16 +589,11 @@ __global__ void __cluster_dims__(CH_CL, 1, 1) __launch_bounds__(CH_THREADS, 2) k
 }
 
 
-bool pow2(float x) {
-    int e;
-    return std::frexp(x, &e) == 0.5f && e > -100 && e < 100;
-}
-
 KFn chain_kernel(int kind, const KArgs &a) {
     const bool w = a.simd == 16;
     if (kind != PH_PRESSURE && a.model != 1) return chain_scalar_kernel(kind, a.model);
     switch (kind) {
-        case PH_PRESSURE: return (pow2(a.dxk) && pow2(a.dyk)) ? k_pressure_chain<true> : k_pressure_chain<false>;
+        case PH_PRESSURE: return (chain_pow2(a.dxk) && chain_pow2(a.dyk)) ? k_pressure_chain<true> : k_pressure_chain<false>;
         case PH_U: return w ? k_mom_chain<COMP_U, 16> : k_mom_chain<COMP_U, 8>;
         case PH_V: return w ? k_mom_chain<COMP_V, 16> : k_mom_chain<COMP_V, 8>;
         default: return w ? k_mom_chain<COMP_W, 16> : k_mom_chain<COMP_W, 8>;
@@ -627,10 +622,19 @@ size_t chain_unit_words(int nii, int njj) {
 
 int chain_claims(int ni) { return (ni + CH_SR * CH_CL - 1) / (CH_SR * CH_CL); }
 
+bool chain_pow2(float x) {
+    int e;
+    return std::frexp(x, &e) == 0.5f && e > -100 && e < 100;
+}
+
 cudaError_t chain_grid(int kind, const KArgs &a, long long claims, int *grid) {
+    return chain_grid_of((const void *)chain_kernel(kind, a), CH_THREADS, claims, grid);
+}
+
+cudaError_t chain_grid_of(const void *kernel, int threads, long long claims, int *grid) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(CH_CL);
-    cfg.blockDim = dim3(CH_THREADS);
+    cfg.blockDim = dim3(threads);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = CH_CL;
@@ -638,7 +642,7 @@ cudaError_t chain_grid(int kind, const KArgs &a, long long claims, int *grid) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int clusters = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, chain_kernel(kind, a), &cfg);
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
     if (e != cudaSuccess) return e;
     *grid = CH_CL * (int)std::max<long long>(1, std::min<long long>(std::max(1, clusters), claims));
     return cudaSuccess;

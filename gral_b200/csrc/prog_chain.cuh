@@ -35,6 +35,9 @@ using KFn = void (*)(KArgs, SweepGeom, ChainBufs);
 KFn chain_scalar_kernel(int kind, int model);
 KFn chain_scalar_terms(int kind, int model);
 int chain_scalar_pairs(int model);
+// grid of a chain kernel: whole clusters, at most one per claim
+cudaError_t chain_grid_of(const void *kernel, int threads, long long claims, int *grid);
+bool chain_pow2(float x);
 
 namespace {
 
@@ -212,7 +215,7 @@ struct ChainSmem {
 // ring 0 (for the sweep's first row: the values the sweep does not change).
 template <class Job, int PH, int SR, int M, int CL, int IS, int JS>
 __device__ __forceinline__ void run_chain(const KArgs &a, const SweepGeom &g, const ChainBufs &b,
-                                          ChainSmem<SR, Job::NV> &sm) {
+                                          ChainSmem<SR, Job::NV> &sm, Job job = Job()) {
     constexpr int NV = Job::NV;                   // values of a column handed to the row below,
     constexpr int NJ = Job::NJ;                   // the first NJ of them also to the row's next column
     constexpr int NF = Job::NF;                   // and the first NF stored in fields
@@ -222,7 +225,6 @@ __device__ __forceinline__ void run_chain(const KArgs &a, const SweepGeom &g, co
     const bool mine = l2 < ks;       // this lane holds levels of the column
     const unsigned rank = cluster_rank();
     const unsigned ring0 = smem_u32(sm.ring) + lane * 16u;
-    Job job;
     job.init(a, lane);
     const unsigned gstamp = (unsigned)*b.epoch * 8u + PH;      // of the words in global memory
     const unsigned units = (unsigned)min(b.unit_n, max(0, *a.nact - b.unit_lo));

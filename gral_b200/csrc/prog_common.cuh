@@ -308,6 +308,7 @@ __device__ inline bool wait_stamps(const int *f1, const int *f2, int stamp, int 
 // APP, ATP, ABP with KKART < k-1 (abp1) and at KKART+1 (abp0), DZK; and the per-situation DTIME.
 struct DiagTabs {
     const float *dzk, *app, *atp, *abp0, *abp1;
+    const float *tab;      // row chains: T, P above KKART+1, P at KKART+1 per level, [3][NKK+2]
     const float *dtime;
 };
 

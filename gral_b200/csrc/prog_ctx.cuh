@@ -121,6 +121,10 @@ struct gral_ctx {
     // DiagnosticFlowfield after the solve (gral_params.post_diagnostic)
     bool post_diag = false;
     int diag_grid = 0;
+    DiagChainBufs dcb{};       // row chains of the diagnostic sweeps (levels 0: not used)
+    DevBuf<float> ddiv;
+    DevBuf<unsigned long long> dwords;
+    DevBuf<int> dstamp;
     DevBuf<float> ddpm, dtab, ddt;
     DevBuf<int> dflags;
     DevBuf<float> varw, z0i;
@@ -164,6 +168,7 @@ struct gral_ctx {
         meta.release(); cflags.release(); colf.release(); sit.release(); colke.release(); rcw.release();
         ddpm.release(); dtab.release(); ddt.release(); dflags.release(); fseg.release();
         varw.release(); z0i.release();
+        ddiv.release(); dwords.release(); dstamp.release();
         crec.release(); cwords.release(); cptab.release(); cint.release();
         gff.release(); gffoff.release(); gffkk.release(); gffu.release(); l2flush.release();
         prep.release();

@@ -505,8 +505,22 @@ int run_diagnostic(gral_ctx *ctx) {
     DiagTabs t;
     t.dzk = ctx->dtab.p; t.app = ctx->dtab.p + nk2; t.atp = ctx->dtab.p + 2 * nk2;
     t.abp0 = ctx->dtab.p + 3 * nk2; t.abp1 = ctx->dtab.p + 4 * nk2;
+    t.tab = ctx->dtab.p + 5 * nk2;
     t.dtime = ctx->ddt.p;
     launch_diag_dtime(kd, ctx->params[0].kadvmax, ctx->ddt.p, st);
+    if (ctx->dcb.levels) {
+        const DiagChainBufs &db = ctx->dcb;
+        CK(cudaMemsetAsync(db.dpm, 0, (size_t)ctx->nb * ctx->ncols * 64 * (db.levels / 2) * sizeof(float), st));
+        CK(cudaMemsetAsync(db.words, 0, ctx->dwords.n * sizeof(unsigned long long), st));
+        for (int d = 1; d <= 10; ++d) {                // Iterations = 10 after a prognostic solve (:33-37)
+            kd.diag_iter = d;
+            CK(cudaMemsetAsync(ctx->counters.p, 0, 8 * kCounterSlots * sizeof(unsigned int), st));
+            launch_diag_chain(kd, ctx->geo_p.g, t, db, st);
+        }
+        launch_diag_wfinal(kd, t, st);
+        CK(cudaGetLastError());
+        return GRAL_OK;
+    }
     CK(cudaMemsetAsync(ctx->ddpm.p, 0, (size_t)ctx->nb * ctx->ncols * nk2 * sizeof(float), st));
     CK(cudaMemsetAsync(ctx->dflags.p, 0, (size_t)ctx->nb * ctx->ncols * sizeof(int), st));
     for (int d = 1; d <= 10; ++d) {                    // Iterations = 10 after a prognostic solve (:33-37)
@@ -997,7 +1011,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
         // full-height level tables of DiagnosticFlowfield.cs:124-138 (float, the reference's
         // expressions): dzk, app, atp, abp0 (k = KKART+1), abp1 (k > KKART+1)
         const float *DZK = s->dzk;
-        std::vector<float> dt(5 * (size_t)nk2, 0.0f);
+        std::vector<float> dt(8 * (size_t)nk2, 0.0f);
         for (int k = 0; k < nk2; ++k) dt[k] = DZK[k];
         for (int k = 1; k <= NKK - 1; ++k) {
             dt[nk2 + k] = 2 * (DYK * DZK[k] / DXK + DXK * DZK[k] / DYK + DXK * DYK / DZK[k]);
@@ -1005,8 +1019,39 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
             dt[3 * nk2 + k] = DXK * DYK / DZK[k];
             dt[4 * nk2 + k] = DXK * DYK / (0.5F * (DZK[k - 1] + DZK[k]));
         }
+        // forward elimination from NKK-1 down, the same in every column: T, P above KKART+1, P at KKART+1
+        float P = 0.0f;
+        for (int k = NKK - 1; k >= 1; --k) {
+            const float T = 1.0f / (dt[nk2 + k] - dt[2 * nk2 + k] * P);
+            P = dt[4 * nk2 + k] * T;
+            dt[5 * nk2 + k] = T;
+            dt[6 * nk2 + k] = P;
+            dt[7 * nk2 + k] = dt[3 * nk2 + k] * T;
+        }
         CK(ctx->dtab.ensure(dt.size()));
-        CK(ctx->ddpm.ensure((size_t)n * ncols * nk2));
+        ctx->dcb = DiagChainBufs{};
+        if (const int lv = diag_chain_levels(NKK)) {
+            // DIV/DTIME for as many situations at a time as fit 4 GB; without memory for the planes the
+            // diagonal-claim wavefront below
+            const size_t unit = (size_t)ncols * 64 * (lv / 2);
+            int units = (int)std::max<size_t>(1, std::min<size_t>(n, ((size_t)4 << 30) / (unit * sizeof(float))));
+            units = std::max(units, (n + kCounterSlots - 1) / kCounterSlots);
+            cudaError_t e = ctx->ddpm.ensure(unit * n);
+            if (e == cudaSuccess) e = ctx->ddiv.ensure(unit * units);
+            if (e == cudaSuccess) e = ctx->dwords.ensure(diag_chain_words(NII, NJJ, lv) * n);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                ctx->ddpm.release(); ctx->ddiv.release(); ctx->dwords.release();
+            } else {
+                CK(e);
+                const int stamps[10] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10};
+                CK(ctx->dstamp.ensure(10));
+                CK(cudaMemcpyAsync(ctx->dstamp.p, stamps, sizeof(stamps), cudaMemcpyHostToDevice, st));
+                ctx->dcb = DiagChainBufs{lv, units, 0, ctx->ddiv.p, ctx->ddpm.p, ctx->dwords.p, ctx->dstamp.p};
+                CK(diag_chain_grid(lv, NII - 2, units, &ctx->dcb.grid));
+            }
+        }
+        if (!ctx->dcb.levels) CK(ctx->ddpm.ensure((size_t)n * ncols * nk2));
         CK(ctx->dflags.ensure((size_t)n * ncols));
         CK(ctx->ddt.ensure(n));
         CK(cudaMemcpyAsync(ctx->dtab.p, dt.data(), dt.size() * sizeof(float), cudaMemcpyHostToDevice, st));

@@ -88,6 +88,18 @@ cudaError_t diag_occupancy(int ks, int *blocks_per_sm);
 void launch_diag_dtime(const KArgs &a, int kadvmax, float *dtime, cudaStream_t st);
 void launch_diag_pressure(const KArgs &a, const SweepGeom &g, const DiagTabs &t, int grid, cudaStream_t st);
 void launch_diag_velcorr(const KArgs &a, const DiagTabs &t, cudaStream_t st);
+// the same sweeps on row chains (prog_chain_diag.cu): one iteration, pressure sweep and velocity
+// correction, on DPM in planes; levels = levels per lane (diag_chain_levels, 0: too many for a warp)
+struct DiagChainBufs {
+    int levels, units, grid;         // units: situations whose DIV/DTIME is held at once
+    float *div, *dpm;                // levels/2 planes [units or all situations][col][64]
+    unsigned long long *words;       // zeroed before the first iteration
+    const int *stamps;               // [iteration-1], distinct
+};
+int diag_chain_levels(int nkk);
+size_t diag_chain_words(int nii, int njj, int levels);   // words of one situation
+cudaError_t diag_chain_grid(int levels, int ni, int units, int *grid);
+void launch_diag_chain(const KArgs &a, const SweepGeom &g, const DiagTabs &t, const DiagChainBufs &buf, cudaStream_t st);
 void launch_diag_wfinal(const KArgs &a, const DiagTabs &t, cudaStream_t st);
 
 }  // namespace gral

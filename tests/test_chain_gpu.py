@@ -91,3 +91,31 @@ def test_batch_on_row_chains_equals_interleaved(gpu_required, monkeypatch, model
         for name in ("uk", "vk", "wk") + (("turb", "tdiss") if model == 2 else ()):
             np.testing.assert_array_equal(getattr(res[0][0][b], name), getattr(res[1][0][b], name), err_msg=(b, name))
         np.testing.assert_array_equal(res[0][1][b], res[1][1][b])
+
+
+@pytest.mark.parametrize("nii,njj,dx,stretch,n,hills", [
+    (6, 5, 2.0, 1.05, 1, False),        # one block, not full
+    (34, 9, 2.5, 1.05, 1, False),       # 32 rows, a spacing that is no power of two
+    (35, 21, 2.0, 1.05, 2, True),       # a second claim of one row, two situations, hills
+    (19, 22, 2.0, 1.01, 2, False),      # 162 levels: six a lane; 17 rows, a second claim of one
+])
+def test_diagnostic_chain_matches_oracle(gpu_required, nii, njj, dx, stretch, n, hills):
+    """The pressure sweeps of the diagnostic step after the solve, on row chains over the full height."""
+    if hills:
+        dom = domain(nii, njj, dx, dx, True)
+    else:
+        dom = prep.make_domain(nii, njj, dx, 2.0, stretch, 14, [prep.Building(3, 4, 3, 4, 7.0)])
+    sits = [prep.random_situation(300 + nii + q) for q in range(n)]
+    ps = [dom.params(x, model=1, iterations=2, post_diagnostic=1) for x in sits]
+    f0 = [prep.initial_fields(dom, x, 1) for x in sits]
+    fg = [f.copy() for f in f0]
+    with PrognosticSolver(dom.nii, dom.njj, dom.nkk, dom.kadvmax, max_batch=n) as s:
+        s.calculate_batch(ps, dom.static, fg)
+        again = [f.copy() for f in f0]
+        s.calculate_batch(ps, dom.static, again)      # the same context once more
+    for b in range(n):
+        fc = f0[b].copy()
+        O.solve(ps[b], dom.static, fc)
+        for name in ("uk", "vk", "wk"):
+            np.testing.assert_array_equal(getattr(fg[b], name), getattr(fc, name), err_msg=(b, name))
+            np.testing.assert_array_equal(getattr(again[b], name), getattr(fc, name), err_msg=(b, name))
