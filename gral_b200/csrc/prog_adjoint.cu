@@ -43,6 +43,7 @@
 #include <cstdlib>
 
 #include "adj_level.cuh"
+#include "prog_chain.cuh"
 #include "prog_ctx.cuh"
 #include "prog_level.cuh"
 
@@ -290,6 +291,11 @@ struct __align__(16) MomShared {
     float rows[NROW][KMAX_LEVELS];
 };
 
+struct LevelSpan {
+    int lo = 0, hi = KMAX_LEVELS;
+    __device__ __forceinline__ bool has(int k) const { return k >= lo && k <= hi; }
+};
+
 template <int COMP>
 struct MomRev {
     const KArgs &a;
@@ -337,15 +343,18 @@ struct MomRev {
         for_inputs<InTab<COMP>::N>([&](auto q) { x[q.value] = input<q.value>(k, IS, JS); });
     }
 
-    // before the wait: the forward rows of the column from the kept states and its Thomas
-    // recurrence (U-prognostic-microscale_1.cs:485-504)
-    __device__ void pre(int i, int j, int IS, int JS) {
-        const int lane = threadIdx.x & 31;
+    __device__ void column(int i, int j) {
         c = make_col(a, i, j);
         act = (c.fl & F_ADV) != 0;
         kkm = (COMP == 0) ? c.kkm_u : (COMP == 1 ? c.kkm_v : -32768);
         kwl = ((c.fl & F_CUTKLT1) && (c.fl & F_Z0GE)) ? c.KK + 2 : c.KK + 1;
         top_carry = 0.0f;
+    }
+
+    // the column and, if it is solved, its forward rows A, B, C, D from the kept states
+    __device__ void rows(int i, int j, int IS, int JS) {
+        const int lane = threadIdx.x & 31;
+        column(i, j);
         if (!act) return;
 #pragma unroll 1
         for (int r = 0; r < 2; ++r) {
@@ -363,6 +372,14 @@ struct MomRev {
             S[R_UP][k] = __ldcg(d.end[COMP] + cell(a, c.col, k + 1));
         }
         __syncwarp();
+    }
+
+    // before the wait: the forward rows of the column and its Thomas recurrence
+    // (U-prognostic-microscale_1.cs:485-504)
+    __device__ void pre(int i, int j, int IS, int JS) {
+        const int lane = threadIdx.x & 31;
+        rows(i, j, IS, JS);
+        if (!act) return;
         if (lane == 0) {
             float P = 0.0f, Q = 0.0f;
             for (int k = c.K0; k <= c.VI; ++k) {
@@ -542,7 +559,9 @@ struct MomRev {
         }
     }
 
-    __device__ void after(int IS, int JS) {
+    // the level cotangents of the row added to every input; s1, s2: the levels at which the two
+    // predecessors have already been given theirs
+    __device__ void after(int IS, int JS, LevelSpan s1 = LevelSpan{}, LevelSpan s2 = LevelSpan{}) {
         if (!act) return;
         const int lane = threadIdx.x & 31;
         constexpr int N = CompTraits<COMP>::N;
@@ -563,8 +582,8 @@ struct MomRev {
                 constexpr InDesc e = InTab<COMP>::at(q.value);
                 const float v = g[q.value];
                 if constexpr (e.f == COMP) {
-                    // the predecessors' cotangents were sent as words
-                    if ((e.di != 0 && e.dj == 0 && e.di == -IS) || (e.di == 0 && e.dj != 0 && e.dj == -JS)) return;
+                    if (e.di != 0 && e.dj == 0 && e.di == -IS && s1.has(k + e.dk)) return;
+                    if (e.di == 0 && e.dj != 0 && e.dj == -JS && s2.has(k + e.dk)) return;
                 }
                 if constexpr (e.f == FVEG) {
                     if (!a.veg) return;
@@ -772,6 +791,8 @@ __global__ void __launch_bounds__(AW * 32) k_adj_pressure(KArgs a, AdjArgs d, Sw
     rev_tasks(a, d, g, IS, JS, job);
 }
 
+#include "adj_chain.cuh"
+
 // which columns' row carry some column reads (bit 0: IS = +1, bit 1: IS = -1); rcr zeroed before
 __global__ void k_adj_readers(KArgs a, int *rcr) {
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
@@ -932,26 +953,27 @@ __device__ __forceinline__ bool div_at(const KArgs &a, int i, int j, int k) {
     return k > m.kkart && k <= m.vi;
 }
 
-__global__ void k_adj_div(KArgs a, AdjArgs d) {
+// raw: L_DIV holds the cotangent of DIM, DIV/DTIME
+__global__ void k_adj_div(KArgs a, AdjArgs d, bool raw) {
     int col, i, j;
     if (!warp_col(a, col, i, j)) return;
     const int lane = threadIdx.x & 31;
     const int nj2 = a.nj2;
     const float *LDV = d.lam[L_DIV];
-    const float AREA = a.areaxy;
+    const float AREA = a.areaxy, dt = raw ? a.sit[0].dtime : 1.0f;
     for (int k = lane; k < a.ks; k += 32) {
         if (k < 1) continue;
         const float dz = a.dzk[k];
         float gu = 0.0f, gv = 0.0f, gw = 0.0f;
         if (div_at(a, i, j, k)) {
-            const float l = LDV[cell(a, col, k)];
+            const float l = LDV[cell(a, col, k)] / dt;
             gu += l * a.dyk * dz;
             gv += l * a.dxk * dz;
             if (k > a.meta[col].kkart + 1) gw += l * AREA;
         }
-        if (div_at(a, i - 1, j, k)) gu -= LDV[cell(a, col - nj2, k)] * a.dyk * dz;
-        if (div_at(a, i, j - 1, k)) gv -= LDV[cell(a, col - 1, k)] * a.dxk * dz;
-        if (div_at(a, i, j, k - 1)) gw -= LDV[cell(a, col, k - 1)] * AREA;
+        if (div_at(a, i - 1, j, k)) gu -= LDV[cell(a, col - nj2, k)] / dt * a.dyk * dz;
+        if (div_at(a, i, j - 1, k)) gv -= LDV[cell(a, col - 1, k)] / dt * a.dxk * dz;
+        if (div_at(a, i, j, k - 1)) gw -= LDV[cell(a, col, k - 1)] / dt * AREA;
         if (gu != 0.0f) d.lam[FU][cell(a, col, k)] += gu;
         if (gv != 0.0f) d.lam[FV][cell(a, col, k)] += gv;
         if (gw != 0.0f) d.lam[FW][cell(a, col, k)] += gw;
@@ -1336,12 +1358,59 @@ int pressure_tables(gral_ctx *ctx) {
     return GRAL_OK;
 }
 
+// segments whose kept states are on the device at a time
+int keep_buffers(int segments) { return segments > 1 ? 2 : 1; }
+
 int rev_grid(gral_ctx *ctx, const SweepGeom &g) {
     const double width = (double)g.ni * g.nj / std::max(1, g.ni + g.nj - 1);
     double la = 12.0;   // diagonals of wavefront width the reverse sweeps keep warps for (6: 12 % slower)
     if (const char *v = std::getenv("GRAL_PROG_ADJ_LOOKAHEAD")) la = std::max(1.0, std::atof(v));
     const long long want = (long long)std::ceil(la * width / AW);
     return (int)std::max<long long>(ctx->num_sms, std::min<long long>(4LL * ctx->num_sms, want));
+}
+
+// The row chains of the reverse sweeps, if the context runs row chains and their buffers can be
+// had; on = false otherwise, and the one-kernel wavefronts run instead.
+int reverse_chains(gral_ctx *ctx, int iterations, RevChains &r, bool &on) {
+    on = false;
+    if (!use_chain(ctx)) return GRAL_OK;
+    const KArgs &a = ctx->ka;
+    const size_t fsz = (size_t)a.ncols * a.ks, words = chain_unit_words(a.nii, a.njj);
+    cudaError_t e = ctx->adj_rec.ensure((size_t)a.ncols * AM_PAIRS * KMAX_LEVELS);
+    if (e == cudaSuccess) e = ctx->adj_plane.ensure(PL_N * fsz);
+    if (e == cudaSuccess) e = ctx->adj_word.ensure(words);
+    if (e == cudaSuccess) e = ctx->adj_int.ensure(2 + (size_t)iterations);
+    if (e == cudaSuccess) e = ctx->adj_sit.ensure(1);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        ctx->adj_rec.release(); ctx->adj_plane.release(); ctx->adj_word.release();
+        return GRAL_OK;
+    }
+    CK(e);
+    cudaStream_t st = ctx->stream;
+    // the unit list (situation 0, active), and a word stamp per reversed iteration over cleared words
+    std::vector<int> v(2 + (size_t)iterations);
+    v[0] = 0;
+    v[1] = 1;
+    for (int q = 0; q < iterations; ++q) v[2 + q] = 1 + q;
+    CK(cudaMemcpyAsync(ctx->adj_int.p, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(ctx->adj_sit.p, a.sit, sizeof(SitDev), cudaMemcpyDeviceToDevice, st));
+    CK(cudaMemcpyAsync(&ctx->adj_sit.p->active, ctx->adj_int.p + 1, sizeof(int), cudaMemcpyDeviceToDevice, st));
+    CK(cudaMemsetAsync(ctx->adj_word.p, 0, words * sizeof(unsigned long long), st));
+    r.a = a;
+    r.a.sit = ctx->adj_sit.p;
+    r.a.act = ctx->adj_int.p;
+    r.a.nact = ctx->adj_int.p + 1;
+    r.a.counters = ctx->adj_ctr.p;
+    r.b = ChainBufs{ctx->adj_rec.p, ctx->adj_word.p, nullptr, ctx->adj_int.p + 2, 0, 1, 0};
+    r.h = AdjChain{ctx->adj_rec.p, ctx->adj_plane.p, ctx->cb.ptab, fsz};
+    CK(chain_grid_of((const void *)k_adj_press_chain, CH_THREADS, chain_claims(ctx->geo_p.g.ni), &r.grid[PH_PRESSURE]));
+    CK(chain_grid_of((const void *)k_adj_mom_chain<0>, CH_THREADS, chain_claims(ctx->geo_u.g.ni), &r.grid[PH_U]));
+    CK(chain_grid_of((const void *)k_adj_mom_chain<1>, CH_THREADS, chain_claims(ctx->geo_v.g.ni), &r.grid[PH_V]));
+    CK(chain_grid_of((const void *)k_adj_mom_chain<2>, CH_THREADS, chain_claims(ctx->geo_p.g.ni), &r.grid[PH_W]));
+    CK(cudaStreamSynchronize(st));     // v leaves scope
+    on = true;
+    return GRAL_OK;
 }
 
 }  // namespace
@@ -1360,7 +1429,7 @@ int gral_prog_vjp_forward(gral_ctx *ctx, const gral_params *p, const gral_static
         return fail(ctx, GRAL_EINVAL, "the adjoint differentiates turbulence model 1, parity width 8, quantise 0");
     if (iterations < 1 || checkpoint_every < 0)
         return fail(ctx, GRAL_EINVAL, "iterations must be >= 1 and checkpoint_every >= 0");
-    ctx->adj_ready = false;
+    ctx->adj_ready = ctx->adj_last_kept = false;
     gral_params q = *p;
     q.iteration_steps_min = iterations;
     q.iteration_steps_max = iterations;
@@ -1391,14 +1460,30 @@ int gral_prog_vjp_forward(gral_ctx *ctx, const gral_params *p, const gral_static
                                     st));
     } else {
         const int nck = (iterations + checkpoint_every - 1) / checkpoint_every;
+        // the last segment is reversed first: its states are kept while it runs, where there is room, and
+        // gral_prog_vjp has nothing to recompute before it starts
+        const size_t buf = keep_buffers(nck) * checkpoint_every, nevk = (size_t)std::max(nev[0] + nev[1], 1) * a.ks;
+        cudaError_t e = ctx->adj_keep.ensure(buf * NKEEP * fsz);
+        if (e == cudaSuccess) e = ctx->adj_bits.ensure(buf * nevk);
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+        else CK(e);
+        const bool keep = e == cudaSuccess;
+        const size_t slot0 = (size_t)((nck - 1) % keep_buffers(nck)) * checkpoint_every;
+        if (keep) CK(cudaMemsetAsync(ctx->adj_bits.p, 0, buf * nevk, st));
         CK(ctx->adj_ckpt.ensure((size_t)nck * NCKPT * fsz));
         CK(ctx->adj_cksit.ensure(nck));
         CK(ctx->adj_ckit.ensure(nck));
         CK(cudaEventRecord(ctx->ev[0], st));
         for (int it = 0; it < iterations; ++it) {
             if (it % checkpoint_every == 0) CK_RC(save_checkpoint(ctx, it / checkpoint_every));
-            CK_RC(forward_iteration(ctx, nullptr, nullptr, st));
+            const int q = it - (nck - 1) * checkpoint_every;     // position in the last segment
+            if (keep && q >= 0)
+                CK_RC(forward_iteration(ctx, ctx->adj_keep.p + (slot0 + q) * NKEEP * fsz,
+                                        ctx->adj_bits.p + (slot0 + q) * nevk, st));
+            else
+                CK_RC(forward_iteration(ctx, nullptr, nullptr, st));
         }
+        ctx->adj_last_kept = keep;
     }
     CK(cudaEventRecord(ctx->ev[1], st));
     CK(cudaGetLastError());
@@ -1411,7 +1496,7 @@ int gral_prog_vjp_forward(gral_ctx *ctx, const gral_params *p, const gral_static
     if (herr == ERR_TIMEOUT) return fail(ctx, GRAL_ETIMEDOUT, "a wavefront wait exceeded its time limit");
     ctx->it_host = iterations + 1;
     CK_RC(gral_prog_store(ctx, f, nullptr));
-    CK_RC(pressure_tables(ctx));
+    if (!use_chain(ctx)) CK_RC(pressure_tables(ctx));
     ctx->adj_iters = iterations;
     ctx->adj_every = checkpoint_every;
     ctx->adj_ready = true;
@@ -1431,19 +1516,27 @@ int gral_prog_vjp(gral_ctx *ctx, const float *dj_duk, const float *dj_dvk, const
     const size_t fsz = (size_t)a.ncols * a.ks, ssz = (size_t)a.ncols * (a.nkk + 2);
     const int nev = ctx->adj_nwe + ctx->adj_nsn;
     const int nseg = (N + K - 1) / K;
-    const int nbuf = nseg > 1 ? 2 : 1;     // the next segment is recomputed while this one is reversed
+    const int nbuf = keep_buffers(nseg);     // the next segment is recomputed while this one is reversed
     // (with all states kept there is one segment, and nothing to recompute)
+    const bool last_kept = ctx->adj_last_kept;
+    if (nseg > nbuf) ctx->adj_last_kept = false;      // this call overwrites its buffer
     const size_t nevk = (size_t)std::max(nev, 1) * a.ks;
     CK(ctx->adj_keep.ensure((size_t)nbuf * K * NKEEP * fsz));
     CK(ctx->adj_lam.ensure((size_t)NLAM * fsz));
     CK(ctx->adj_stg.ensure(3 * ssz));
-    CK(ctx->adj_slot.ensure(2 * (size_t)a.ncols * a.ks));
     CK(ctx->adj_rcr.ensure(a.ncols));
-    CK(ctx->adj_ctr.ensure(4));
+    CK(ctx->adj_ctr.ensure(8));
     CK(ctx->adj_bits.ensure((size_t)nbuf * K * nevk));
     CK(cudaMemsetAsync(ctx->adj_lam.p, 0, (size_t)NLAM * fsz * sizeof(float), st));
-    CK(cudaMemsetAsync(ctx->adj_slot.p, 0, 2 * (size_t)a.ncols * a.ks * sizeof(unsigned long long), st));
-    if (!all) CK(cudaMemsetAsync(ctx->adj_bits.p, 0, (size_t)nbuf * K * nevk, st));
+    RevChains rc;
+    bool chains = false;
+    CK_RC(reverse_chains(ctx, N, rc, chains));
+    if (!chains) {
+        if (use_chain(ctx)) CK_RC(pressure_tables(ctx));
+        CK(ctx->adj_slot.ensure(2 * (size_t)a.ncols * a.ks));
+        CK(cudaMemsetAsync(ctx->adj_slot.p, 0, 2 * (size_t)a.ncols * a.ks * sizeof(unsigned long long), st));
+    }
+    if (!all && !last_kept) CK(cudaMemsetAsync(ctx->adj_bits.p, 0, (size_t)nbuf * K * nevk, st));
     if (!ctx->adj_stream) CK(cudaStreamCreateWithFlags(&ctx->adj_stream, cudaStreamNonBlocking));
     cudaStream_t st2 = ctx->adj_stream;
     StageLam L{ctx->adj_stg.p, ctx->adj_stg.p + ssz, ctx->adj_stg.p + 2 * ssz};
@@ -1480,7 +1573,7 @@ int gral_prog_vjp(gral_ctx *ctx, const float *dj_duk, const float *dj_dvk, const
     auto recompute = [&](int sg) -> int {
         if (sg + nbuf < nseg) CK(cudaStreamWaitEvent(st2, E(sg + nbuf, 3), 0));   // that buffer's last reader
         CK(cudaEventRecord(E(sg, 0), st2));
-        if (!all) {
+        if (!all && !(last_kept && sg == nseg - 1)) {
             CK_RC(restore_checkpoint(ctx, sg, st2));
             const int n = std::min(K, N - sg * K);
             for (int q = 0; q < n; ++q) CK_RC(forward_iteration(ctx, keep_of(sg, q), bits_of(sg, q), st2));
@@ -1502,24 +1595,35 @@ int gral_prog_vjp(gral_ctx *ctx, const float *dj_duk, const float *dj_dvk, const
             for (int f = 0; f < 3; ++f) d.end[f] = kp + (7 + f) * fsz;
             d.bits = bits_of(sg, q);
             d.it = it0 + q + 1;
-            CK(cudaMemsetAsync(d.ctr, 0, 4 * sizeof(unsigned int), st));
-            d.stamp = ++stamp;
-            k_adj_mom<2><<<g_p, AW * 32, 0, st>>>(a, d, ctx->geo_p.g);
-            d.ctr = ctx->adj_ctr.p + 1;
-            d.stamp = ++stamp;
-            k_adj_mom<1><<<g_v, AW * 32, 0, st>>>(a, d, ctx->geo_v.g);
-            d.ctr = ctx->adj_ctr.p + 2;
-            d.stamp = ++stamp;
-            k_adj_mom<0><<<g_u, AW * 32, 0, st>>>(a, d, ctx->geo_u.g);
+            CK(cudaMemsetAsync(d.ctr, 0, 8 * sizeof(unsigned int), st));
+            if (chains) {
+                rc.b.epoch = ctx->adj_int.p + 2 + (d.it - 1);
+                launch_adj_mom<2>(rc, d, ctx->geo_p.g, st);
+                launch_adj_mom<1>(rc, d, ctx->geo_v.g, st);
+                launch_adj_mom<0>(rc, d, ctx->geo_u.g, st);
+            } else {
+                d.stamp = ++stamp;
+                k_adj_mom<2><<<g_p, AW * 32, 0, st>>>(a, d, ctx->geo_p.g);
+                d.ctr = ctx->adj_ctr.p + 1;
+                d.stamp = ++stamp;
+                k_adj_mom<1><<<g_v, AW * 32, 0, st>>>(a, d, ctx->geo_v.g);
+                d.ctr = ctx->adj_ctr.p + 2;
+                d.stamp = ++stamp;
+                k_adj_mom<0><<<g_u, AW * 32, 0, st>>>(a, d, ctx->geo_u.g);
+            }
             k_adj_avg_copies<<<cb, 256, 0, st>>>(a, d);
             k_adj_avg_gather<<<cb, 256, 0, st>>>(a, d);
             k_adj_avg_clear<<<cb, 256, 0, st>>>(a, d);
             k_adj_velcorr<<<cb, 256, 0, st>>>(a, d);
-            d.ctr = ctx->adj_ctr.p + 3;
-            d.stamp = ++stamp;
-            k_adj_pressure<<<g_p, AW * 32, 0, st>>>(a, d, ctx->geo_p.g);
-            d.ctr = ctx->adj_ctr.p;
-            k_adj_div<<<cb, 256, 0, st>>>(a, d);
+            if (chains) {
+                launch_adj_pressure(rc, d, ctx->geo_p.g, st);
+            } else {
+                d.ctr = ctx->adj_ctr.p + 3;
+                d.stamp = ++stamp;
+                k_adj_pressure<<<g_p, AW * 32, 0, st>>>(a, d, ctx->geo_p.g);
+                d.ctr = ctx->adj_ctr.p;
+            }
+            k_adj_div<<<cb, 256, 0, st>>>(a, d, chains);
             k_adj_bc_top_rev<<<(a.ncols + 127) / 128, 128, 0, st>>>(a, d);
             const long long ns = (long long)(a.nii - 1) * a.ks, nw = (long long)(a.njj - 1) * a.ks;
             k_adj_bc_sn_rev<<<(int)((ns + 127) / 128), 128, 0, st>>>(a, ctx->bc, d);

@@ -150,6 +150,7 @@ struct gral_ctx {
     // discrete adjoint (gral_prog_vjp_forward / gral_prog_vjp): checkpoints of the forward state,
     // the states kept for one checkpoint segment, cotangent fields, reverse-sweep words
     bool adj_ready = false;
+    bool adj_last_kept = false;   // the last segment's states are in adj_keep
     int adj_iters = 0, adj_every = 0, adj_nwe = 0, adj_nsn = 0;
     double adj_ms_forward = 0.0;
     DevBuf<float> adj_ckpt, adj_keep, adj_lam, adj_ptab, adj_stg;
@@ -159,6 +160,12 @@ struct gral_ctx {
     DevBuf<unsigned long long> adj_slot;   // stamped cotangent words of the reverse sweeps
     DevBuf<int> adj_rcr;                   // per column: whose row carry some column reads
     DevBuf<uint8_t> adj_bits;
+    // row chains of the reverse sweeps: records, level fields, words, unit list and epochs, active situation
+    DevBuf<float2> adj_rec;
+    DevBuf<float> adj_plane;
+    DevBuf<unsigned long long> adj_word;
+    DevBuf<int> adj_int;
+    DevBuf<SitDev> adj_sit;
     cudaStream_t adj_stream = nullptr;   // recomputation of the next segment beside the reverse sweeps
 
     ~gral_ctx() {
@@ -176,6 +183,7 @@ struct gral_ctx {
         counters.release();
         adj_ckpt.release(); adj_keep.release(); adj_lam.release(); adj_ptab.release(); adj_stg.release();
         adj_cksit.release(); adj_ckit.release(); adj_ctr.release(); adj_slot.release(); adj_rcr.release(); adj_bits.release();
+        adj_rec.release(); adj_plane.release(); adj_word.release(); adj_int.release(); adj_sit.release();
         for (auto &e : ev) if (e) cudaEventDestroy(e);
         if (adj_stream) cudaStreamDestroy(adj_stream);
         if (stream) cudaStreamDestroy(stream);

@@ -125,3 +125,43 @@ def test_vjp_rejects_other_configurations_and_order(gpu_required):
         with pytest.raises(GralError) as e:   # a negative checkpoint spacing
             s.vjp_forward(p, dom.static, f.copy(), 3, -1)
         assert e.value.code == GRAL_EINVAL
+
+
+@pytest.mark.parametrize("nii,njj,dx,dy,hills", [
+    (6, 5, 2.0, 2.0, False),        # 4 and 3 sweep rows: one block of a row chain, not full for U
+    (7, 40, 2.5, 2.5, False),       # 5 and 4 rows
+    (34, 9, 2.0, 4.0, False),       # 32 and 31 rows: one claim, full and not
+    (35, 33, 3.0, 2.0, True),       # 33 and 32 rows: a second claim of one row; row carries
+    (67, 21, 2.0, 2.5, True),       # 65 and 64 rows: three claims and two
+])
+def test_vjp_on_row_chains(gpu_required, monkeypatch, nii, njj, dx, dy, hills):
+    """The reverse sweeps as row chains against the FP64 tape (the bound of the tape test above) and
+    against the one-kernel wavefronts that run without row chains.  The two round differently at up to
+    four operations of a column step (4 * 6e-8); a step's influence fades within a few columns
+    (factor 3), and five iterations have twenty sweeps: 1.5e-5, bound 2e-5.  Five iterations cover the
+    four sweep directions."""
+    if hills:
+        dom = prep.hilly_domain(nii, njj, dx, 18, seed=nii, n_hills=2, n_buildings=3)
+    else:
+        dom = prep.make_domain(nii, njj, dx, 2.0, 1.05, 18, [prep.Building(3, 4, 3, 4, 7.0)], dyk=dy)
+    sit = prep.random_situation(700 + nii)
+    f = prep.initial_fields(dom, sit)
+    n = 5
+    p = dom.params(sit, model=1, iterations=n, quantise=0)
+    rng = np.random.default_rng(nii)
+    g = [rng.normal(size=f.uk.shape).astype(np.float32).astype(np.float64) for _ in range(3)]
+    x0 = tuple(x.astype(np.float64) for x in (f.uk, f.vk, f.wk))
+    veg = np.zeros(f.uk.shape) if dom.static.veg is None else dom.static.veg.astype(np.float64)
+    ref = O.twin_vjp(p, dom.static, f, x0, veg, n, g)
+    monkeypatch.setenv("GRAL_PROG_PLAIN_MODE", "0")
+    wave = gpu_vjp(dom, p, f, n, 2, g)[1]
+    monkeypatch.setenv("GRAL_PROG_PLAIN_MODE", "6")
+    with PrognosticSolver(dom.nii, dom.njj, dom.nkk, dom.kadvmax) as s:
+        s.vjp_forward(p, dom.static, f.copy(), n, 2)
+        chain = s.vjp(*(a.astype(np.float32) for a in g))
+        # again: the last segment's kept states have been overwritten and are recomputed
+        again = s.vjp(*(a.astype(np.float32) for a in g))
+    for q in range(3):
+        assert rel_l2(chain[1 + q], ref[q]) <= 2e-3
+        assert rel_l2(chain[1 + q], wave[1 + q]) <= 2e-5
+        assert rel_l2(again[1 + q], chain[1 + q]) <= 1e-5
