@@ -182,7 +182,7 @@ __device__ __forceinline__ void mom_dir(int it, int &IS, int &JS) {
 }
 
 template <int COMP>
-__global__ void __launch_bounds__(AC_BLOCK * 32) k_adj_mom_terms(KArgs a, AdjArgs d, SweepGeom g, AdjChain h) {
+__global__ void __launch_bounds__(AC_BLOCK * 32, 5) k_adj_mom_terms(KArgs a, AdjArgs d, SweepGeom g, AdjChain h) {
     __shared__ MomShared sm[AC_BLOCK];
     MomShared &M = sm[threadIdx.x >> 5];
     int IS, JS, i1, j1, i, j;
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(AC_BLOCK * 32) k_adj_mom_terms(KArgs a, AdjArg
 }
 
 template <int COMP>
-__global__ void __launch_bounds__(AC_BLOCK * 32) k_adj_mom_rest(KArgs a, AdjArgs d, SweepGeom g, AdjChain h) {
+__global__ void __launch_bounds__(AC_BLOCK * 32, 5) k_adj_mom_rest(KArgs a, AdjArgs d, SweepGeom g, AdjChain h) {
     __shared__ MomShared sm[AC_BLOCK];
     MomShared &M = sm[threadIdx.x >> 5];
     int IS, JS, i1, j1, i, j;
