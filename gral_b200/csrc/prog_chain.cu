@@ -130,6 +130,7 @@ __device__ __forceinline__ void level_rec(LevelRec &r, const MomPre &p, int IS, 
 // of the block's eight warps waiting).
 template <int COMP, int SW>
 __global__ void __launch_bounds__(CT_THREADS, 4) k_mom1_terms(KArgs a, SweepGeom g, ChainBufs b) {
+    grid_wait();
     __shared__ float sA[CT_COLS][KMAX_LEVELS + 1], sB[CT_COLS][KMAX_LEVELS + 1], sC[CT_COLS][KMAX_LEVELS + 1];
     __shared__ ColCtx s_col[CT_COLS];
     __shared__ float s_ust[CT_COLS];
@@ -226,6 +227,7 @@ __global__ void __launch_bounds__(CT_THREADS, 4) k_mom1_terms(KArgs a, SweepGeom
 // level of PT_COLS columns, all operands loaded before a column's flags decide anything.
 constexpr int PT_COLS = 2;
 __global__ void __launch_bounds__(256) k_pressure_terms(KArgs a, ChainBufs b) {
+    grid_wait();
     const int u = blockIdx.y, k = threadIdx.x, ks = a.ks;
     if (b.unit_lo + u >= *a.nact) return;
     const int s = a.act[b.unit_lo + u];
@@ -657,9 +659,9 @@ void launch_chain(int kind, const KArgs &a, const SweepGeom &g, const ChainBufs 
         const long long tiles = (long long)n * g.ni * ((g.nj + CT_COLS - 1) / CT_COLS);
         if (kind == PH_PRESSURE) {
             const int rows = std::max(1, 256 / a.ks), per = rows * PT_COLS;
-            k_pressure_terms<<<dim3((a.ncols + per - 1) / per, n), dim3(a.ks, rows), 0, st>>>(a, b);
+            launch_after(k_pressure_terms, dim3((a.ncols + per - 1) / per, n), dim3(a.ks, rows), st, a, b);
         } else {
-            terms_kernel(kind, a)<<<(unsigned)tiles, CT_THREADS, 0, st>>>(a, g, b);
+            launch_after(terms_kernel(kind, a), (unsigned)tiles, CT_THREADS, st, a, g, b);
         }
         chain_kernel(kind, a)<<<grid, CH_THREADS, 0, st>>>(a, g, b);
     }

@@ -133,6 +133,7 @@ __device__ __forceinline__ void neighbours(const MomPre &p, int IS, int JS, floa
 
 template <int MODEL, int COMP>
 __global__ void __launch_bounds__(CT_THREADS, 3) k_scal_terms(KArgs a, SweepGeom g, ChainBufs b) {
+    grid_wait();
     constexpr bool Z = MODEL == 0 && COMP == COMP_W, DIFF = MODEL == 2;
     constexpr int NP = Z ? (int)Z_PAIRS : scal_pairs<MODEL, COMP>(), KL = KMAX_LEVELS;
     __shared__ float sA[CT_COLS][KL + 1], sB[CT_COLS][KL + 1], sC[CT_COLS][KL + 1];
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_scal_terms(KArgs a, SweepGeom
 // Coefficients of the k-eps sweep.  A level with a wall function (and one at or below KKART) is a
 // constant of the sweep: its value goes into the record and nothing updates it.
 __global__ void __launch_bounds__(CT_THREADS, 2) k_tke_terms(KArgs a, SweepGeom g, ChainBufs b) {
+    grid_wait();
     constexpr int KL = KMAX_LEVELS;
     __shared__ float sm_f[5][CT_COLS][KL + 1];     // A, B1, C1, B2, C2
     __shared__ TileSmem sm;

@@ -220,6 +220,18 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
 __device__ __forceinline__ void st_release(int *p, int v) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// The light launches of a slab iteration are set up while the launch before them runs (launch_after):
+// their kernels first wait until it has completed and its writes are visible, then let the launch
+// after them be set up.  Every thread block waits before it touches global memory, so a kernel's end implies the
+// end of all before it; without the attribute both calls do nothing.  The row chains are launched after
+// their coefficients' end, and nothing starts beside them: set up early their
+// clusters share SMs (400x400: 2.77 ms an iteration; 2.63 this way, 2.64 with plain launches; 16x14: 123, 129,
+// 143 us).
+__device__ __forceinline__ void grid_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -79,6 +79,7 @@ __device__ __forceinline__ void col_loop(const KArgs &a, bool need_active, Body 
 // the reference's sequential i loop; rows and levels are independent.
 template <bool IL>
 __global__ void k_bc_we(KArgs a, BcLists bc) {
+    grid_wait();
     const int j = 2 + blockIdx.x * blockDim.y + threadIdx.y;
     if (j > a.njj) return;
     int s, kbeg, kstep;
@@ -119,6 +120,7 @@ __global__ void k_bc_we(KArgs a, BcLists bc) {
 
 template <bool IL>
 __global__ void k_bc_sn(KArgs a, BcLists bc) {
+    grid_wait();
     const int i = 2 + blockIdx.x * blockDim.y + threadIdx.y;
     if (i > a.nii) return;
     int s, kbeg, kstep;
@@ -214,6 +216,7 @@ __device__ __forceinline__ bool make_cells(const KArgs &a, CellGrid &c) {
 // which stores DPM only), the update of DPMNEW and the residual maximum (:877-893)
 template <bool PRESS>
 __global__ void __launch_bounds__(256) k_velcorr_cell(KArgs a) {
+    grid_wait();
     CellGrid c;
     if (!make_cells(a, c)) return;
     const SitDev &sd = a.sit[c.s];
@@ -267,6 +270,7 @@ __global__ void __launch_bounds__(256) k_velcorr_cell(KArgs a) {
 
 // staggered -> cell-centre averages of one level (average_col)
 __global__ void __launch_bounds__(256) k_average_cell(KArgs a) {
+    grid_wait();
     CellGrid c;
     if (!make_cells(a, c)) return;
     const int ks = a.ks, nj2 = a.nj2, k = c.k;
@@ -320,6 +324,7 @@ __global__ void __launch_bounds__(256) k_average_cell(KArgs a) {
 
 // top: level VerticalIndex copied to VerticalIndex+1, a thread per column (a warp per column: 53 -> 14 us)
 __global__ void __launch_bounds__(128) k_bc_top_cell(KArgs a) {
+    grid_wait();
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= a.ncols || (int)blockIdx.y >= *a.nact) return;
     const int s = a.act[blockIdx.y], i = col / a.nj2, j = col - i * a.nj2;
@@ -341,6 +346,7 @@ __global__ void k_average_b(KArgs a) {
 
 // ---- convergence bookkeeping (:1144-1178), one thread per situation ----
 __global__ void k_bookkeeping(KArgs a) {
+    grid_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) {
         *a.it_global += 1;   // kernels of this launch read SitDev::it, never it_global
@@ -593,25 +599,26 @@ void launch_bc(const KArgs &a, const BcLists &bc, cudaStream_t st) {
         k_bc_sn<true><<<dim3((a.nii - 1 + 7) / 8, units), blk, 0, st>>>(a, bc);
     } else {
         k_bc_we<false><<<dim3((a.njj - 1 + 7) / 8, units), blk, 0, st>>>(a, bc);
-        k_bc_sn<false><<<dim3((a.nii - 1 + 7) / 8, units), blk, 0, st>>>(a, bc);
+        launch_after(k_bc_sn<false>, dim3((a.nii - 1 + 7) / 8, units), blk, st, a, bc);
     }
     if (a.il) k_bc_top_b<<<col_grid<true>(a), COL_WARPS * 32, 0, st>>>(a);
-    else k_bc_top_cell<<<dim3((a.ncols + 127) / 128, a.nb), 128, 0, st>>>(a);
+    else launch_after(k_bc_top_cell, dim3((a.ncols + 127) / 128, a.nb), 128, st, a);
 }
 
 void launch_velcorr(const KArgs &a, cudaStream_t st) {
     if (a.il) k_velcorr_b<<<col_grid<true>(a), COL_WARPS * 32, 0, st>>>(a);
-    else if (a.chain) k_velcorr_cell<true><<<cell_grid(a), cell_block(a), 0, st>>>(a);
-    else k_velcorr_cell<false><<<cell_grid(a), cell_block(a), 0, st>>>(a);
+    else if (a.chain) launch_after(k_velcorr_cell<true>, cell_grid(a), cell_block(a), st, a);
+    else launch_after(k_velcorr_cell<false>, cell_grid(a), cell_block(a), st, a);
 }
 
 void launch_average(const KArgs &a, cudaStream_t st) {
     if (a.il) k_average_b<<<col_grid<true, true>(a), COL_WARPS * 32, 0, st>>>(a);
-    else k_average_cell<<<cell_grid(a), cell_block(a), 0, st>>>(a);
+    else launch_after(k_average_cell, cell_grid(a), cell_block(a), st, a);
 }
 
 void launch_bookkeeping(const KArgs &a, cudaStream_t st) {
-    k_bookkeeping<<<(a.nb + 127) / 128, 128, 0, st>>>(a);
+    if (a.il) k_bookkeeping<<<(a.nb + 127) / 128, 128, 0, st>>>(a);
+    else launch_after(k_bookkeeping, (a.nb + 127) / 128, 128, st, a);
 }
 
 void launch_setup(const KArgs &a, const Staging &sg, int model, const float *varw, const float *z0_init,

@@ -22,6 +22,21 @@ struct Staging {
     size_t stride;   // floats between situations
 };
 
+// A launch that is set up while the launch before it on the stream runs (its kernel calls grid_wait first).
+template <class... P, class... A>
+void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, const A &...args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Buffers of the row-chain schedule (prog_chain.cu): column records of the units in flight, stamped
 // words between claims, the pressure sweep's elimination table per i-direction.
 struct ChainBufs {
