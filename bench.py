@@ -51,6 +51,7 @@ import argparse
 import json
 import math
 import os
+import select
 import statistics
 import subprocess
 import sys
@@ -157,7 +158,9 @@ def profile_traffic(layout: str, phase: str, cells: int):
 
 
 class ClockSampler:
-    """nvidia-smi clocks and throttle reasons sampled every 200 ms during the timed region."""
+    """nvidia-smi clocks and throttle reasons sampled every 20 ms during the timed region, which can
+    be as short as 50 ms.  Entering waits (5 s at most) for the first sample, so nvidia-smi is up; that
+    one, taken before the region, is not counted."""
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
          "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
          "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
@@ -169,8 +172,10 @@ class ClockSampler:
     def __enter__(self):
         try:
             self.proc = subprocess.Popen(["nvidia-smi", "-i", str(self.dev), f"--query-gpu={self.Q}",
-                                          "--format=csv,noheader,nounits", "-lms", "200"],
-                                         stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
+                                          "--format=csv,noheader,nounits", "-lms", "20"],
+                                         stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True, bufsize=1)
+            if select.select([self.proc.stdout], [], [], 5.0)[0]:
+                self.proc.stdout.readline()
         except Exception:
             self.proc = None
         return self
