@@ -7,11 +7,14 @@
 // between the columns (two per column, contractions as in the forward, see prog_chain.cuh); a
 // parallel kernel turns the row's cotangents into those of its inputs.
 //
-// What bounds it: the chain of (rows + columns) column steps, then the scattered float atomics of the last
-// kernel.  The one-kernel wavefront (rev_tasks) paid a hand-off through global memory and about 100 levels of
-// serial recurrence per diagonal, 3.1 us of each; this runs 1.0 us steps of a row in shared memory.
+// What bounds it: in the chain the column steps, 0.41 us each (a wavefront step of rev_tasks, a hand-off
+// through global memory and about 100 levels of serial recurrence, took 3.1 us); in the parallel kernels
+// latency: 55-60 % of the issue slots stay empty behind 32-35 loads a level at 16-20 warps an SM.  200x200, levels 25, us of a
+// momentum sweep: terms 165, chain 163, rest 170 (rev_tasks 1250); pressure: 12, 221 (1250).
 
-constexpr int AC_BLOCK = 4;     // warps (columns) of a block of the parallel kernels
+// Warps (columns) of a block of the parallel kernels.  Their five blocks an SM (96 registers, a few spilled)
+// measured 21.5 ms for the reverse of 12 iterations on 200x200, four without spills 22.6, six 21.9, eight 23.6.
+constexpr int AC_BLOCK = 4;
 constexpr int AM_PAIRS = 3, AP_PAIRS = 2;
 
 struct AdjChain {

@@ -14,17 +14,19 @@
 // the W sweep ("end") and the branch taken by every lateral boundary copy, then reverses the
 // segment's iterations one by one.  Reversing one iteration (PrognosticFlowfield.cs:584-1137):
 //
-//   W, V, U momentum sweeps   reverse Gauss-Seidel wavefronts: a column receives the cotangents
-//                             of its new values from its two sweep successors (stamped 8-byte
-//                             words), reverses the relaxed back-substitution and the Thomas
-//                             recurrence (U-prognostic-microscale_1.cs:485-524) on lane 0, sends
-//                             its two predecessors the cotangents of their new values the same
-//                             way, and then adds the per-level vector-Jacobian products of the
-//                             coefficient assembly (adj_level.cuh) to every other input;
+//   W, V, U momentum sweeps   reverse Gauss-Seidel sweeps: a column receives the cotangents of its
+//                             new values from its two sweep successors, reverses the relaxed
+//                             back-substitution and the Thomas recurrence
+//                             (U-prognostic-microscale_1.cs:485-524), hands its two predecessors the
+//                             cotangents of their new values, and adds the per-level vector-Jacobian
+//                             products of the coefficient assembly (adj_level.cuh) to every other
+//                             input.  Row chains (adj_chain.cuh) wherever the context runs them and
+//                             their buffers fit; otherwise one wavefront kernel per sweep (rev_tasks:
+//                             stamped 8-byte words through global memory, recurrences on lane 0);
 //   staggered averages        gathers (PrognosticFlowfield.cs:958-1039);
 //   velocity correction       a gather into DPM (PrognosticFlowfield.cs:904-949);
-//   pressure correction       a reverse wavefront of the transposed tridiagonal solves
-//                             (PrognosticFlowfield.cs:804-901), the row carry of Q included;
+//   pressure correction       a reverse sweep of the transposed tridiagonal solves in the same two
+//                             forms (PrognosticFlowfield.cs:804-901), the row carry of Q included;
 //   divergence                a gather (PrognosticFlowfield.cs:723-758);
 //   boundary conditions       the copies reversed in reverse order (PrognosticFlowfield.cs:595-714).
 //

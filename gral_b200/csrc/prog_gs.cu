@@ -13,6 +13,9 @@
 // Values another warp may write inside the same kernel (the swept field, the pressure row carry)
 // are read with ld.global.cg so no stale L1 line is used.
 //
+// The slab family's sweeps run as row chains (prog_chain.cu) by default; its wavefronts here, on diagonal
+// claims and on strips of rows, run where the chains' buffers do not fit or another mode is asked for.
+//
 // Two families share the per-level arithmetic of prog_level.cuh:
 //   plain   (slab layout)        one warp per (situation, column), lane = level; lane 0 runs the
 //                                serial Thomas sweep on the warp's shared rows;

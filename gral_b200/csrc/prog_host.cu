@@ -433,8 +433,8 @@ int tune_variants(gral_ctx *ctx) {
 }
 
 // Schedule of the slab family's sweeps.  The row chains are the fastest on every grid measured
-// (ms of an iteration, row chains / best other: 16x14 0.17 / 0.24, 100x100 0.60 / 1.53, 200x200 1.33 /
-// 3.54, 400x400 3.38 / 8.33), so they run wherever their buffers fit.  Otherwise the diagonal-claim
+// (ms of an iteration, row chains / best other: 16x14 0.13 / 0.24, 100x100 0.51 / 1.53, 200x200 1.18 /
+// 3.54, 400x400 2.63 / 8.33), so they run wherever their buffers fit.  Otherwise the diagonal-claim
 // wavefront and the strip variants, which give bit-identical results, each run two live iterations
 // before the first convergence test (the first warms the kernels up), the second timed with CUDA
 // events, and the fastest is kept and captured into the iteration graph; without room for the trials

@@ -119,7 +119,7 @@ typedef struct gral_stats {
     float *trace_delta_umax;     /* optional, caller-owned: DeltaUMax per iteration */
     int32_t trace_capacity;
     double ms_total, ms_upload, ms_iterate, ms_download;
-    int32_t layout;              /* device layout used: 0 slab (one warp per column), 1 interleaved
+    int32_t layout;              /* device layout used: 0 slab (columns contiguous), 1 interleaved
                                     (32 situations per group, one block per group-column) */
     int32_t launch_variant;      /* launch variant the autotuner kept: interleaved layout, the batched
                                     kernels' variant; slab layout, the schedule of the sweeps
