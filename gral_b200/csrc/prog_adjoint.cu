@@ -47,6 +47,7 @@
 #include "adj_level.cuh"
 #include "prog_chain.cuh"
 #include "prog_ctx.cuh"
+#include "prog_pages.cuh"
 #include "prog_level.cuh"
 
 namespace gral {
@@ -1634,6 +1635,9 @@ int gral_prog_vjp(gral_ctx *ctx, const float *dj_duk, const float *dj_dvk, const
         CK(cudaEventRecord(E(sg, 3), st));
         CK(cudaGetLastError());
     }
+    // while the GPU reverses: pages for the results
+    first_touch({{dj_dveg, ssz * sizeof(float)}, {dj_duk0, ssz * sizeof(float)}, {dj_dvk0, ssz * sizeof(float)},
+                 {dj_dwk0, ssz * sizeof(float)}});
     CK(cudaStreamSynchronize(st));
     CK(cudaStreamSynchronize(st2));
     float ms_re = 0.f, ms_rev = 0.f;

@@ -8,6 +8,7 @@
 #include <cstring>
 
 #include "prog_ctx.cuh"
+#include "prog_pages.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -399,6 +400,7 @@ int gral_prog_gff_pack(gral_ctx *ctx, int32_t situation, int32_t mode, float win
     CK(cudaGetLastError());
     int hbad = 0;
     if (mode == GRAL_GFF_TKE) CK(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+    first_touch({{out + GRAL_GFF_HEADER_BYTES, 2 * (size_t)words}});
     CK(cudaMemcpyAsync(out + GRAL_GFF_HEADER_BYTES, ctx->gff.p, 2 * (size_t)words, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (hbad) return fail(ctx, GRAL_ENONFINITE, "non-finite TKE value: the reference's conversion fails there");
@@ -502,6 +504,7 @@ int gral_prog_gff_unpack(gral_ctx *ctx, const uint8_t *payload, uint64_t bytes, 
     CK(cudaMemsetAsync(du, 0, 3 * cells * sizeof(float), st));
     launch_gff_unpack(g, flag, ctx->gff.p, ctx->gffkk.p, ctx->gffoff.p, du, dv, dw, st);
     CK(cudaGetLastError());
+    first_touch({{uk, cells * sizeof(float)}, {vk, cells * sizeof(float)}, {wk, cells * sizeof(float)}});
     CK(cudaMemcpyAsync(uk, du, cells * sizeof(float), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(vk, dv, cells * sizeof(float), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(wk, dw, cells * sizeof(float), cudaMemcpyDeviceToHost, st));

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "prog_ctx.cuh"
+#include "prog_pages.cuh"
 #include "prog_prep.cuh"
 
 namespace gral {
@@ -446,6 +447,7 @@ int gral_prog_flat_init(gral_ctx *ctx, const gral_flat_grid *g, const float *cut
     int *d_kadv = nullptr;
     rc = flat_fill(ctx, g, b.cutk.p, b.adv.p, dzk, hokart, met, du, dv, dw, &d_kadv, true);
     if (rc != GRAL_OK) return rc;
+    first_touch({{f->uk, cells * sizeof(float)}, {f->vk, cells * sizeof(float)}, {f->wk, cells * sizeof(float)}});
     int kadv1 = 1;
     CK(cudaMemcpyAsync(&kadv1, d_kadv, 4, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(kkart, b.kkart.p, ncols * sizeof(int16_t), cudaMemcpyDeviceToHost, st));
@@ -532,6 +534,7 @@ int gral_prog_vegetation(gral_ctx *ctx, int32_t nii, int32_t njj, int32_t nkk, c
                                                              b.kkart.p, d_dzk, d_hok, b.veg.p, b.mask.p, b.cov.p);
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[1], st));
+    first_touch({{veg, cells * sizeof(float)}});
     CK(cudaMemcpyAsync(veg, b.veg.p, cells * sizeof(float), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(veg_mask, b.mask.p, ncols, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(cov, b.cov.p, ncols * sizeof(float), cudaMemcpyDeviceToHost, st));

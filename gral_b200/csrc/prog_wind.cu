@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "prog_ctx.cuh"
+#include "prog_pages.cuh"
 
 namespace gral {
 
@@ -192,6 +193,8 @@ extern "C" int gral_prog_wind_at(gral_ctx *ctx, int32_t situation, const gral_wi
         a, n, reinterpret_cast<const gral_particle *>(b.points.p), d_u, d_v, d_w, b.ints.p, d_bad);
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[1], st));
+    const size_t nb = (size_t)n * 4;
+    first_touch({{ux, nb}, {uy, nb}, {uz, nb}, {index_k, nb}});
     int hbad = 0;
     CK(cudaMemcpyAsync(&hbad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(ux, d_u, (size_t)n * 4, cudaMemcpyDeviceToHost, st));

@@ -281,7 +281,10 @@ class PrognosticSolver:
         cutk, dzk, hokart = (np.ascontiguousarray(a, np.float32) for a in (cutk, dzk, hokart))
         adv = None if advdom is None else np.ascontiguousarray(advdom, np.uint8)
         shape = (nii + 2, njj + 2, nkk + 2)
-        f = FieldArrays(*(np.empty(shape, np.float32) for _ in range(3)))
+        # one block for the three fields: the C library keeps a freed block for the next call as long as what
+        # is free at the top of its heap is below twice the largest block freed, so with three blocks
+        # and VEG it gave the pages back and every call faulted them in again
+        f = FieldArrays(*np.empty((3,) + shape, np.float32))
         kk = np.empty((nii + 2, njj + 2), np.int16)
         ahk = np.empty((nii + 2, njj + 2), np.float32)
         kadv = C.c_int32()
@@ -313,8 +316,8 @@ class PrognosticSolver:
         the stored fields of `situation` as Zeitschleife.IntWindCalculate does."""
         p = np.ascontiguousarray(particles, dtype=PARTICLE_DTYPE)
         n = p.size
-        ux, uy, uz = (np.empty(n, np.float32) for _ in range(3))
-        kk = np.empty(n, np.int32)
+        out = np.empty((4, n), np.float32)     # one block, as in flat_init
+        ux, uy, uz, kk = out[0], out[1], out[2], out[3].view(np.int32)
         m = None if met is None else met.to_c()
         g = GralWindGrid(grid.get("terrain", 0), grid.get("buildings", 1), grid.get("ikooa", 0), grid.get("jkooa", 0),
                          grid["dxk"], grid["dyk"], grid.get("ahmin", 0.0),
