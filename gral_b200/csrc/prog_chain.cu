@@ -422,7 +422,7 @@ struct MomChain {
             const bool more = __any_sync(0xffffffffu, differ(nQ, inQ));
             inU = nU; inQ = nQ;
             down();
-            if (!more) break;      // Q is final, and this round used it
+            if (!more) break;      // Q is final and has been used
             up();
         }
         for (;;) {
@@ -538,7 +538,7 @@ struct PressChain {
             const bool more = __any_sync(0xffffffffu, differ(nQ, inQ));
             inD = nD; inQ = nQ;
             up();
-            if (!more) break;      // Q is final, and this round used it
+            if (!more) break;      // Q is final and has been used
             down();
         }
         for (;;) {
