@@ -655,6 +655,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
     ctx->il = il;
     ctx->ngroups = ngroups;
     ctx->loaded = false;
+    ctx->adj_ready = ctx->adj_last_kept = false;    // the checkpoints are of the load before
     drop_graph(ctx);
     ctx->stored = false;
     ctx->h_kkart.assign(s->kkart, s->kkart + (size_t)ncols);
