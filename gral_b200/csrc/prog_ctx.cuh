@@ -11,6 +11,7 @@
 #include "gral_prog.h"
 #include "prog_common.cuh"
 #include "prog_kernels.cuh"
+#include "unit_sets.h"
 
 namespace gral {
 
@@ -46,8 +47,6 @@ struct PrepBufs {
         ints.release(); kkart.release(); adv.release(); mask.release(); points.release();
     }
 };
-
-constexpr int kCounterSlots = 64;   // wavefront launches per phase (group sets) with own counters
 
 struct Geom {
     SweepGeom g;

@@ -553,18 +553,16 @@ int reserve_chain(gral_ctx *ctx) {
     cudaStream_t st = ctx->stream;
     const size_t unit = chain_record_bytes(ctx->model) * ctx->ncols;
     const size_t words = chain_unit_words(ctx->nii, ctx->njj);
-    int units = (int)std::max<size_t>(1, std::min<size_t>(ctx->nb, kChainBytes / unit));
-    if (const char *v = std::getenv("GRAL_PROG_CHAIN_UNITS")) units = std::max(1, std::min(units, std::atoi(v)));
-    units = std::max(units, (ctx->nb + kCounterSlots - 1) / kCounterSlots);
-    const int sets = (ctx->nb + units - 1) / units;
-    units = (ctx->nb + sets - 1) / sets;              // sets of equal size
+    size_t fit = kChainBytes / unit;
+    if (const char *v = std::getenv("GRAL_PROG_CHAIN_UNITS")) fit = std::min(fit, (size_t)std::max(1, std::atoi(v)));
+    int units = set_units(ctx->nb, fit);
     const size_t had = ctx->cwords.n;
     const int had_int = (int)ctx->cint.n;
     constexpr int kPasses = 8;     // flags of the table's passes, reused round by round
     cudaError_t e = ctx->crec.ensure(unit / sizeof(float2) * units);
-    while (e == cudaErrorMemoryAllocation && units > std::max(1, (ctx->nb + kCounterSlots - 1) / kCounterSlots)) {
+    for (int less; e == cudaErrorMemoryAllocation && (less = fewer_units(ctx->nb, units)) > 0;) {
         cudaGetLastError();
-        units = (units + 1) / 2;
+        units = less;
         e = ctx->crec.ensure(unit / sizeof(float2) * units);
     }
     if (e == cudaSuccess) e = ctx->cwords.ensure(words * ctx->nb);
@@ -1042,8 +1040,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
             // DIV/DTIME for as many situations at a time as fit 4 GB; without memory for the planes the
             // diagonal-claim wavefront below
             const size_t unit = (size_t)ncols * 64 * (lv / 2);
-            int units = (int)std::max<size_t>(1, std::min<size_t>(n, ((size_t)4 << 30) / (unit * sizeof(float))));
-            units = std::max(units, (n + kCounterSlots - 1) / kCounterSlots);
+            const int units = set_units(n, ((size_t)4 << 30) / (unit * sizeof(float)));
             cudaError_t e = ctx->ddpm.ensure(unit * n);
             if (e == cudaSuccess) e = ctx->ddiv.ensure(unit * units);
             if (e == cudaSuccess) e = ctx->dwords.ensure(diag_chain_words(NII, NJJ, lv) * n);
