@@ -3,8 +3,8 @@
 //
 // Their recurrences divide by A - C*P at every level (U-prognostic-microscale_2.cs:247-256).  The
 // divisor does not depend on the sweep, so its reciprocal is in the record and a quotient is the
-// correctly rounded form of prog_level.cuh (5 dependent operations instead of a division); a column
-// in which a dividend or divisor leaves that form's range is redone with divisions.
+// correctly rounded form of prog_quot.cuh (5 dependent operations instead of a division); a column
+// in which a dividend, quotient or divisor leaves that form's range is redone with divisions.
 #include "prog_chain.cuh"
 
 namespace gral {
@@ -22,43 +22,16 @@ enum : int { Z_CI, Z_CJ, Z_KI, Z_KJ, Z_T1, Z_T2, Z_PHI, Z_FL, Z_C, Z_A, Z_N, Z_D
 enum : int { T_CI, T_CJ, T_KI1, T_KJ1, T_KI2, T_KJ2, T_T1, T_T2, T_T3, T_S1, T_S2, T_FL, T_C1, T_DEN1, T_Y1, T_P1, T_C2, T_DEN2, T_Y2, T_P2, T_K, T_E, T_N };
 constexpr int TKE_PAIRS = T_N / 2;
 
-// level flags: Q recurrence, updated, viscous terms, divisor outside the quotient's range
-enum : unsigned { L_Q = 1u, L_U = 2u, L_X = 4u, L_D = 8u };
+// level flags: Q recurrence, updated, viscous terms, divisor outside the quotient's range; Q in use: the level
+// is updated or, from KKART+1 on (which a taller neighbour keeps from being updated), the next one's Q reads it
+enum : unsigned { L_Q = 1u, L_U = 2u, L_X = 4u, L_D = 8u, L_R = 16u };
+// a level's quot_worst as far as its Q is in use, with the divisor's flag on top
+__device__ __forceinline__ unsigned in_use(unsigned w, unsigned fl) { return (fl & L_R) ? (w | (fl & L_D) << 28) : 0u; }
 
 template <int I>
 __device__ __forceinline__ float lev_a(const float4 *f) { return (I & 1) ? f[I / 2].y : f[I / 2].x; }
 template <int I>
 __device__ __forceinline__ float lev_b(const float4 *f) { return (I & 1) ? f[I / 2].w : f[I / 2].z; }
-
-__device__ __forceinline__ bool odd_divisor(float d) {
-    return (__float_as_uint(d) & 0x7f800000u) - 0x21800000u >= 0x3c000000u;     // outside 2^-60 .. 2^60
-}
-// a dividend that the quotient does not take (zero it does)
-__device__ __forceinline__ bool odd_dividend(float x) {
-    return x != 0.0f && (__float_as_uint(x) & 0x7f800000u) - 0x0d800000u >= 0x62800000u;
-}
-// q = x/d where `on`, with y = RN(1/d); the last operation and the zero case are predicated
-__device__ __forceinline__ void quot_if(float &q, float x, float d, float y, unsigned on) {
-    float q1 = x * y;
-    q1 = fmaf(fmaf(-d, q1, x), y, q1);
-    const float r = fmaf(-d, q1, x);
-    asm("{\n\t.reg .pred f, n;\n\tsetp.ne.u32 f, %5, 0;\n\tsetp.neu.and.f32 n, %1, 0f00000000, f;\n\t"
-        "@f mov.f32 %0, %1;\n\t@n fma.rn.f32 %0, %2, %3, %4;\n\t}"
-        : "+f"(q)
-        : "f"(x), "f"(r), "f"(y), "f"(q1), "r"(on));
-}
-__device__ __forceinline__ void quot_if(double &q, double x, double d, double y, unsigned on) {
-    double q1 = x * y;
-    q1 = fma(fma(-d, q1, x), y, q1);
-    const double r = fma(-d, q1, x);
-    asm("{\n\t.reg .pred f, n;\n\tsetp.ne.u32 f, %5, 0;\n\tsetp.neu.and.f64 n, %1, 0d0000000000000000, f;\n\t"
-        "@f mov.f64 %0, %1;\n\t@n fma.rn.f64 %0, %2, %3, %4;\n\t}"
-        : "+d"(q)
-        : "d"(x), "d"(r), "d"(y), "d"(q1), "r"(on));
-}
-__device__ __forceinline__ bool odd_dividend(double x) {
-    return x != 0.0 && (unsigned)(__double2hiint(x) & 0x7ff00000) - 0x07b00000u >= 0x70000000u;     // 2^-900 .. 2^892
-}
 
 // ------------------------------------ coefficients ------------------------------------------
 
@@ -158,7 +131,8 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_scal_terms(KArgs a, SweepGeom
         float cI, cJ, kI, kJ;
         neighbours(p, t.IS, t.JS, sI, sJ, cI, cJ, kI, kJ);
         const int kkm = COMP == COMP_U ? c.kkm_u : (COMP == COMP_V ? c.kkm_v : -1);
-        const float fl = __uint_as_float((k > c.KK + 1 ? L_Q : 0u) | (k > kkm ? L_U : 0u) | ((DIFF && k > c.KK + 1) ? L_X : 0u));
+        const float fl = __uint_as_float((k > c.KK + 1 ? L_Q : 0u) | (k > kkm ? L_U : 0u) | ((DIFF && k > c.KK + 1) ? L_X : 0u) |
+                                         ((k > c.KK || k > kkm) ? L_R : 0u));
         auto put = [&](int q, float v0, float v1) { rec[q * KL] = make_float2(v0, v1); };
         put(S_CI / 2, cI, cJ);
         put(S_KI / 2, kI, kJ);
@@ -248,7 +222,7 @@ __global__ void __launch_bounds__(CT_THREADS, 2) k_tke_terms(KArgs a, SweepGeom 
         float kI2 = cs * a.tdiss[x.at(dI, k)], kJ2 = ct * a.tdiss[x.at(dJ, k)];
         if (t.IS == -1 && t.JS == -1) { kI1 = kI1 + kJ1; kI2 = kI2 + kJ2; }
         float kn = p.k1, en = p.e1;
-        unsigned fl = k > c.KK + 1 ? L_Q : 0u;
+        unsigned fl = (k > c.KK + 1 ? L_Q : 0u) | (k > c.KK ? L_R : 0u);
         if (k > c.KK) {
             const float *vf[3] = {a.uk, a.vk, a.wk};
             if (tke_wall(a, c, a.colke[c.col], k, kn, en, [&](int f, long long dc, int kk) { return vf[f][x.at(dc, kk)]; })) {
@@ -451,10 +425,22 @@ struct ScalChain {
             if (!more) break;
             up();
         }
-        // dividends of the settled Q (levels the sweep does not change have no say)
+        // dividends and quotients of the settled Q, where they are in use
         const float xa = qA ? Da + A.C * inQ : Da, xb = qB ? Db + B.C * Qa : Db;
-        const bool odd = ((uA | qA) && (odd_dividend(xa) || (A.fl & L_D))) || ((uB | qB) && (odd_dividend(xb) || (B.fl & L_D)));
-        if (__any_sync(0xffffffffu, odd)) {
+        const bool odd = max(in_use(quot_worst(xa, Qa), A.fl), in_use(quot_worst(xb, Qb), B.fl)) >= QUOT_SPAN;
+        // the vote's result is looked at only after the back-substitution, whose rounds hide it
+        const bool redo = __any_sync(0xffffffffu, odd);
+        auto settle = [&]() {
+            for (;;) {
+                const float nU = __shfl_down_sync(0xffffffffu, va, 1);
+                const bool more = __any_sync(0xffffffffu, differ(nU, inU));
+                inU = nU;
+                down();
+                if (!more) break;
+            }
+        };
+        settle();
+        if (redo) {
             Qa = Da / A.den;
             Qb = Db / B.den;
             for (bool first = true;; first = false) {
@@ -467,13 +453,7 @@ struct ScalChain {
             }
             inU = __shfl_down_sync(0xffffffffu, va, 1);
             down();
-        }
-        for (;;) {
-            const float nU = __shfl_down_sync(0xffffffffu, va, 1);
-            const bool more = __any_sync(0xffffffffu, differ(nU, inU));
-            inU = nU;
-            down();
-            if (!more) break;
+            settle();
         }
         Val o;
         o.v[0] = make_float2(va, vb);
@@ -556,9 +536,23 @@ struct W0Chain {
             up();
         }
         const double xa = (double)Da + Ca * inQ, xb = (double)Db + Cb * Qa;
-        auto odd_div = [](double d) { return (unsigned)(__double2hiint(d) & 0x7ff00000) - 0x38000000u >= 0x10000000u; };
-        const bool odd = (qA && (odd_dividend(xa) || odd_div(dA))) || (qB && (odd_dividend(xb) || odd_div(dB)));
-        if (__any_sync(0xffffffffu, odd)) {
+        const unsigned wA = quot_worst(xa, Qa) | (odd_divisor(dA) ? 0x80000000u : 0u);
+        const unsigned wB = quot_worst(xb, Qb) | (odd_divisor(dB) ? 0x80000000u : 0u);
+        const bool odd = max(qA ? wA : 0u, qB ? wB : 0u) >= QUOT_SPAN_DOUBLE;
+        const bool redo = __any_sync(0xffffffffu, odd);
+        auto settle = [&]() {
+            inU = __shfl_down_sync(0xffffffffu, va, 1);
+            down();
+            for (;;) {
+                const float nU = __shfl_down_sync(0xffffffffu, va, 1);
+                const bool more = __any_sync(0xffffffffu, differ(nU, inU));
+                inU = nU;
+                down();
+                if (!more) break;
+            }
+        };
+        settle();
+        if (redo) {
             for (bool first = true;; first = false) {
                 const double nQ = __shfl_up_sync(0xffffffffu, Qb, 1);
                 const bool more = __any_sync(0xffffffffu, !same(nQ, inQ));
@@ -567,15 +561,7 @@ struct W0Chain {
                 if (qA) Qa = ((double)Da + Ca * inQ) / dA;
                 if (qB) Qb = ((double)Db + Cb * Qa) / dB;
             }
-        }
-        inU = __shfl_down_sync(0xffffffffu, va, 1);
-        down();
-        for (;;) {
-            const float nU = __shfl_down_sync(0xffffffffu, va, 1);
-            const bool more = __any_sync(0xffffffffu, differ(nU, inU));
-            inU = nU;
-            down();
-            if (!more) break;
+            settle();
         }
         Val o;
         o.v[0] = make_float2(va, vb);
@@ -678,14 +664,29 @@ struct TkeChain {
             up(0);
             up(1);
         }
-        bool odd = false;
+        unsigned worst = 0;
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
             const float xa = qA ? Da[v] + Ca[v] * inQ[v] : Da[v], xb = qB ? Db[v] + Cb[v] * Qa[v] : Db[v];
-            odd |= ((uA | qA) && odd_dividend(xa)) || ((uB | qB) && odd_dividend(xb));
+            worst = max(worst, max(in_use(quot_worst(xa, Qa[v]), la), in_use(quot_worst(xb, Qb[v]), lb)));
         }
-        odd |= ((uA | qA) && (la & L_D)) || ((uB | qB) && (lb & L_D));
-        if (__any_sync(0xffffffffu, odd)) {
+        const bool redo = __any_sync(0xffffffffu, worst >= QUOT_SPAN);
+        auto settle = [&]() {
+            for (;;) {
+                float nV[2];
+#pragma unroll
+                for (int v = 0; v < 2; ++v) nV[v] = __shfl_down_sync(0xffffffffu, va[v], 1);
+                const bool more = __any_sync(0xffffffffu, differ(nV[0], inV[0]) || differ(nV[1], inV[1]));
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    inV[v] = nV[v];
+                    down(v);
+                }
+                if (!more) break;
+            }
+        };
+        settle();
+        if (redo) {
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
                 Qa[v] = Da[v] / dA[v];
@@ -701,18 +702,7 @@ struct TkeChain {
                 inV[v] = __shfl_down_sync(0xffffffffu, va[v], 1);
                 down(v);
             }
-        }
-        for (;;) {
-            float nV[2];
-#pragma unroll
-            for (int v = 0; v < 2; ++v) nV[v] = __shfl_down_sync(0xffffffffu, va[v], 1);
-            const bool more = __any_sync(0xffffffffu, differ(nV[0], inV[0]) || differ(nV[1], inV[1]));
-#pragma unroll
-            for (int v = 0; v < 2; ++v) {
-                inV[v] = nV[v];
-                down(v);
-            }
-            if (!more) break;
+            settle();
         }
         Val o;
 #pragma unroll

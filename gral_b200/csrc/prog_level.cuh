@@ -12,6 +12,7 @@
 #pragma once
 
 #include "prog_common.cuh"
+#include "prog_quot.cuh"
 
 namespace gral {
 
@@ -112,33 +113,6 @@ __device__ __forceinline__ float pl1(bool v512, float D, float Pe, float Fs) {
 template <int SW>
 __device__ __forceinline__ bool simd16(const KArgs &a) {
     return SW == 0 ? a.simd == 16 : SW == 16;
-}
-
-// Correctly rounded quotients without the compiler's range checks and their branches: with y = RN(1/d),
-// q1 = q0 + (x - d*q0)*y is within an ulp of x/d and RN(q1 + (x - d*q1)*y) is the IEEE quotient
-// (P. Markstein, IBM J. Res. Dev. 34(1), 1990), while no remainder leaves the subnormal range and
-// nothing overflows; a non-finite x gives NaN.  rcp_rn is the reciprocal of a divisor in [2^-27, 2^43):
-// one Newton step on the hardware's approximation, compared with 1/d for every significand at every
-// exponent of that range.  A quotient costs 5 operations, three of a level's faces share a divisor.
-__device__ __forceinline__ float rcp_rn(float d) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
-    return fmaf(fmaf(-d, y, 1.0f), y, y);
-}
-__device__ __forceinline__ float quot(float x, float d, float y) {
-    float q = x * y;
-    q = fmaf(fmaf(-d, q, x), y, q);
-    return fmaf(fmaf(-d, q, x), y, q);
-}
-
-// x/d with y = RN(1/d) for any x: the quotient above where its conditions hold, zero as it is, and the
-// plain division for the rest (magnitudes outside 2^-100 .. 2^97, non-finite values).
-__device__ __forceinline__ float div_by(float x, float d, float y) {
-    const unsigned e = __float_as_uint(x) & 0x7f800000u;
-    const bool zero = x == 0.0f;
-    if (!zero && e - 0x0d800000u >= 0x62800000u) return x / d;
-    const float q = quot(x, d, y);
-    return zero ? x : q;
 }
 
 // sqrt of a sum of squares; zero is kept off the square root's slow path
