@@ -1376,7 +1376,7 @@ int rev_grid(gral_ctx *ctx, const SweepGeom &g) {
 // had; on = false otherwise, and the one-kernel wavefronts run instead.
 int reverse_chains(gral_ctx *ctx, int iterations, RevChains &r, bool &on) {
     on = false;
-    if (!use_chain(ctx)) return GRAL_OK;
+    if (!use_chain(ctx) || !(ctx->chains & 4)) return GRAL_OK;
     const KArgs &a = ctx->ka;
     const size_t fsz = (size_t)a.ncols * a.ks, words = chain_unit_words(a.nii, a.njj);
     cudaError_t e = ctx->adj_rec.ensure((size_t)a.ncols * AM_PAIRS * KMAX_LEVELS);

@@ -75,7 +75,7 @@ struct gral_ctx {
     // strips, then V, W on strip variant 0 (-1: not tuned yet)
     int pmode = -1;
     int fstrip_grid = 0;       // grid of the fused strip launch
-    // row-chain schedule (plain mode 2+strip_num_variants(), model 1): buffers and grids
+    // row-chain schedule (plain mode 2+strip_num_variants(), every model): buffers and grids
     bool chain_ok = false;     // the loaded grid's records and words fit on the device
     int chain_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // indexed by PH_*
     ChainBufs cb{};
@@ -84,6 +84,7 @@ struct gral_ctx {
     DevBuf<float2> cptab;
     DevBuf<int> cint;          // iteration epoch, flags of the elimination table's passes
     int forced_pmode = -1;     // GRAL_PROG_PLAIN_MODE
+    int chains = 7;            // GRAL_PROG_CHAINS: 1 the solver's sweeps, 2 the diagnostic's, 4 the adjoint's reverse sweeps
     int strip_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // indexed by PH_*
     float ptune_ms[16] = {0};  // autotuner timings per plain mode
     std::string err = "no error";

@@ -459,7 +459,7 @@ int tune_plain(gral_ctx *ctx) {
     const int forced_nv = kChainMode() + (ctx->chain_ok ? 1 : 0);
     const int first_stop = std::min(((ctx->it_host + ctx->cadence - 1) / ctx->cadence) * ctx->cadence, ctx->it_max);
     if (ctx->model != 1) {
-        ctx->pmode = ctx->chain_ok ? kChainMode() : 0;
+        ctx->pmode = (ctx->chain_ok && ctx->forced_pmode != 0) ? kChainMode() : 0;
     } else if (ctx->forced_pmode >= 0 && ctx->forced_pmode < forced_nv) {
         ctx->pmode = ctx->forced_pmode;
     } else if (ctx->chain_ok) {
@@ -549,7 +549,7 @@ constexpr size_t kChainBytes = (size_t)16 << 30;
 int reserve_chain(gral_ctx *ctx) {
     ctx->chain_ok = false;
     ctx->ka.epoch = nullptr;
-    if (ctx->il) return GRAL_OK;
+    if (ctx->il || !(ctx->chains & 1)) return GRAL_OK;
     cudaStream_t st = ctx->stream;
     const size_t unit = chain_record_bytes(ctx->model) * ctx->ncols;
     const size_t words = chain_unit_words(ctx->nii, ctx->njj);
@@ -618,6 +618,7 @@ int gral_prog_create(int32_t nii, int32_t njj, int32_t nkk, int32_t kadvmax, int
     }
     if (const char *v = std::getenv("GRAL_PROG_BATCH_VARIANT")) ctx->forced_variant = std::atoi(v);
     if (const char *v = std::getenv("GRAL_PROG_PLAIN_MODE")) ctx->forced_pmode = std::atoi(v);
+    if (const char *v = std::getenv("GRAL_PROG_CHAINS")) ctx->chains = std::atoi(v);
     if (const char *v = std::getenv("GRAL_PROG_LOOKAHEAD")) ctx->lookahead = std::max(0, std::atoi(v));
     if (const char *v = std::getenv("GRAL_PROG_LOOKAHEAD_P")) ctx->lookahead_p = std::max(0, std::atoi(v));
     if (const char *v = std::getenv("GRAL_PROG_LOOKAHEAD_F")) ctx->lookahead_f = std::max(0, std::atoi(v));
@@ -1036,7 +1037,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
         }
         CK(ctx->dtab.ensure(dt.size()));
         ctx->dcb = DiagChainBufs{};
-        if (const int lv = diag_chain_levels(NKK)) {
+        if (const int lv = (ctx->chains & 2) ? diag_chain_levels(NKK) : 0) {
             // DIV/DTIME for as many situations at a time as fit 4 GB; without memory for the planes the
             // diagonal-claim wavefront below
             const size_t unit = (size_t)ncols * 64 * (lv / 2);
