@@ -192,6 +192,35 @@ struct gral_ctx {
 
 namespace gral {
 
+// Element counts of the device buffers of a load whose size depends on the grid, in load_buffers' order: those
+// that gral_prog_load allocates as counted, then the event and task lists (upper bounds) and the buffers
+// of the row chains and the diagnostic step.
+enum : int {
+    LB_SLAB, LB_STAGE, LB_META, LB_CFLAGS, LB_COLF, LB_RCW, LB_COLKE, LB_VARW, LB_Z0I, LB_FLAGS, LB_ROWCARRY, LB_TRACE, LB_VEG, LB_BASE,
+    LB_BCL = LB_BASE, LB_DIAG, LB_FSEG, LB_REC, LB_WORDS, LB_PTAB, LB_DDPM, LB_DDIV, LB_DWORDS, LB_DFLAGS, LB_N
+};
+struct LoadSize {
+    size_t n[LB_N] = {};
+    void cover(const LoadSize &o) {
+        for (int q = 0; q < LB_N; ++q) n[q] = std::max(n[q], o.n[q]);
+    }
+};
+template <class F>
+void load_buffers(gral_ctx &c, F &&f) {
+    f(LB_SLAB, c.slab); f(LB_STAGE, c.stage); f(LB_META, c.meta); f(LB_CFLAGS, c.cflags); f(LB_COLF, c.colf);
+    f(LB_RCW, c.rcw); f(LB_COLKE, c.colke); f(LB_VARW, c.varw); f(LB_Z0I, c.z0i); f(LB_FLAGS, c.flags);
+    f(LB_ROWCARRY, c.rowcarry); f(LB_TRACE, c.trace); f(LB_VEG, c.veg);
+    f(LB_BCL, c.bcl); f(LB_DIAG, c.diag); f(LB_FSEG, c.fseg);
+    f(LB_REC, c.crec); f(LB_WORDS, c.cwords); f(LB_PTAB, c.cptab);
+    f(LB_DDPM, c.ddpm); f(LB_DDIV, c.ddiv); f(LB_DWORDS, c.dwords); f(LB_DFLAGS, c.dflags);
+}
+// counts of a load of n situations in this context (prog_host.cu)
+LoadSize load_size(const gral_ctx *ctx, int n, const gral_params &p, bool veg);
+// device bytes of these counts, as the allocator hands them out
+size_t load_bytes(gral_ctx *ctx, const LoadSize &z);
+// allocates them before the first load, so that loads within these counts allocate nothing large
+int reserve_load(gral_ctx *ctx, const LoadSize &z);
+
 // Slab family, model 1: keep the default schedule of the sweeps (or GRAL_PROG_PLAIN_MODE) without
 // trial iterations, and size its grids (prog_host.cu).
 int plain_schedule_default(gral_ctx *ctx);

@@ -189,6 +189,10 @@ bool interleaved_pays(int n, int nii, int njj, int model) {
     return P[model] * n * cols > A[model] * (nii + njj) + B[model] * groups * cols;
 }
 
+bool interleaved(const gral_ctx *ctx, int n, const gral_params &p) {
+    return ctx->il_min_batch > 0 ? n >= ctx->il_min_batch : interleaved_pays(n, p.nii, p.njj, p.turbulence_model);
+}
+
 int validate(gral_ctx *ctx, int n, const gral_params *p, const gral_static *s, const gral_fields *f) {
     if (!ctx) return GRAL_EINVAL;
     if (n < 1 || n > ctx->cap_batch) return fail(ctx, GRAL_EINVAL, "batch size outside 1..max_batch");
@@ -228,6 +232,9 @@ int validate(gral_ctx *ctx, int n, const gral_params *p, const gral_static *s, c
     return GRAL_OK;
 }
 
+// bounds of the column records that the row chains hold at once and of the diagnostic step's DIV/DTIME
+constexpr size_t kChainBytes = (size_t)16 << 30, kDiagBytes = (size_t)4 << 30;
+
 // the plain mode of the row-chain schedule, after the fused strips
 int kChainMode() { return 2 + strip_num_variants(); }
 
@@ -245,6 +252,68 @@ int gral::strip_variant_of(const gral_ctx *ctx) {
 
 bool gral::fused_strips(const gral_ctx *ctx) {
     return use_strips(ctx) && ctx->pmode == 1 + strip_num_variants();
+}
+
+LoadSize gral::load_size(const gral_ctx *ctx, int n, const gral_params &p, bool veg) {
+    const bool il = interleaved(ctx, n, p);
+    const size_t ncols = (size_t)(p.nii + 2) * (p.njj + 2), nk2 = p.nkk + 2, nj2 = p.njj + 2;
+    const size_t ks = (size_t)((p.kadvmax + 2) + 7) / 8 * 8, groups = (n + 31) / 32, units = il ? groups * 32 : n;
+    const bool ke = p.turbulence_model != 1;
+    LoadSize z;
+    z.n[LB_SLAB] = 10 * units * ncols * ks;
+    z.n[LB_STAGE] = (ke ? 5 : 3) * (size_t)n * ncols * nk2;
+    z.n[LB_META] = z.n[LB_CFLAGS] = z.n[LB_COLF] = z.n[LB_RCW] = ncols;
+    if (ke) {
+        z.n[LB_COLKE] = z.n[LB_Z0I] = ncols;
+        z.n[LB_VARW] = (size_t)n * ncols;
+    }
+    z.n[LB_FLAGS] = (il ? groups : n) * ncols;
+    z.n[LB_ROWCARRY] = units * nj2 * 2 * ks;
+    z.n[LB_TRACE] = (size_t)n * p.iteration_steps_max;
+    if (veg) z.n[LB_VEG] = ncols * ks;
+    z.n[LB_BCL] = 2 * ncols + p.nii + p.njj + 16;
+    z.n[LB_DIAG] = 3 * (size_t)(p.nii + p.njj);
+    z.n[LB_FSEG] = 8 * (size_t)(p.nii + p.njj + 64);
+    if (!il && (ctx->chains & 1)) {
+        z.n[LB_REC] = chain_record_bytes(p.turbulence_model) / sizeof(float2) * ncols * set_units(n, kChainBytes / (chain_record_bytes(p.turbulence_model) * ncols));
+        z.n[LB_WORDS] = chain_unit_words(p.nii, p.njj) * n;
+        z.n[LB_PTAB] = 2 * ncols * ks;
+    }
+    if (p.post_diagnostic) {
+        z.n[LB_DFLAGS] = (size_t)n * ncols;
+        if (const int lv = (ctx->chains & 2) ? diag_chain_levels(p.nkk) : 0) {
+            const size_t unit = ncols * 64 * (lv / 2);
+            z.n[LB_DDPM] = unit * n;
+            z.n[LB_DDIV] = unit * set_units(n, kDiagBytes / (unit * sizeof(float)));
+            z.n[LB_DWORDS] = diag_chain_words(p.nii, p.njj, lv) * n;
+        } else {
+            z.n[LB_DDPM] = (size_t)n * ncols * nk2;
+        }
+    }
+    return z;
+}
+
+size_t gral::load_bytes(gral_ctx *ctx, const LoadSize &z) {
+    // blocks of 1 MB and more come in steps of 2 MB, smaller ones share such a step; 4 MB for those and
+    // the small tables
+    size_t sum = (size_t)4 << 20;
+    load_buffers(*ctx, [&](int q, auto &buf) {
+        const size_t b = z.n[q] * sizeof(*buf.p), step = b >= ((size_t)1 << 20) ? (size_t)2 << 20 : 512;
+        sum += (b + step - 1) / step * step;
+    });
+    return sum;
+}
+
+int gral::reserve_load(gral_ctx *ctx, const LoadSize &z) {
+    cudaError_t e = cudaSuccess;
+    const size_t had = ctx->cwords.n;
+    load_buffers(*ctx, [&](int q, auto &buf) {
+        if (e == cudaSuccess && z.n[q]) e = buf.ensure(z.n[q]);
+    });
+    CK(e);
+    if (ctx->cwords.n != had)      // as reserve_chain leaves new words
+        CK(cudaMemsetAsync(ctx->cwords.p, 0, ctx->cwords.n * sizeof(unsigned long long), ctx->stream));
+    return GRAL_OK;
 }
 
 bool gral::use_chain(const gral_ctx *ctx) { return !ctx->il && ctx->pmode == kChainMode(); }
@@ -544,8 +613,6 @@ int run_diagnostic(gral_ctx *ctx) {
 // situations are independent, so sets of them run one after the other), the words between strips and
 // the elimination table of the pressure sweep, built here.  If they do not fit on the device the
 // strip schedule, which needs none of them, stays the default.
-constexpr size_t kChainBytes = (size_t)16 << 30;
-
 int reserve_chain(gral_ctx *ctx) {
     ctx->chain_ok = false;
     ctx->ka.epoch = nullptr;
@@ -649,7 +716,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
     const int ks = ((p0.kadvmax + 2) + 7) / 8 * 8;
     // Layout: batches for which it is the faster one use the interleaved layout and the
     // lane-per-situation kernels, the others the slab layout and the row chains.
-    const bool il = ctx->il_min_batch > 0 ? n >= ctx->il_min_batch : interleaved_pays(n, NII, NJJ, p0.turbulence_model);
+    const bool il = interleaved(ctx, n, p0);
     const int ngroups = (n + 31) / 32;
     ctx->il = il;
     ctx->ngroups = ngroups;
@@ -862,32 +929,23 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
     const size_t ssz = (size_t)ncols * nk2;
     const int nstage = (ctx->model != 1) ? 5 : 3;
     const int tcap = ctx->it_max;
-    CK(ctx->slab.ensure(fsz * nfields));
-    CK(ctx->stage.ensure(ssz * nstage * n));
-    CK(ctx->meta.ensure(ncols));
-    CK(ctx->cflags.ensure(ncols));
-    CK(ctx->colf.ensure(ncols));
-    CK(ctx->rcw.ensure(ncols));
-    if (ctx->model != 1) {
-        CK(ctx->colke.ensure(ncols));
-        CK(ctx->varw.ensure((size_t)n * ncols));
-        CK(ctx->z0i.ensure(ncols));
-    }
+    const bool has_veg = s->veg && s->veg_mask;
+    const LoadSize z = load_size(ctx, n, p0, has_veg);
+    cudaError_t ze = cudaSuccess;
+    load_buffers(*ctx, [&](int q, auto &buf) {
+        if (q < LB_BASE && ze == cudaSuccess) ze = buf.ensure(z.n[q]);
+    });
+    CK(ze);
     CK(ctx->tables.ensure(7 * ks));
     CK(ctx->ap0.ensure((size_t)n * ks));
     CK(ctx->sit.ensure(n));
     const size_t flag_units = il ? (size_t)ngroups : (size_t)n;
-    CK(ctx->flags.ensure(flag_units * ncols));
-    CK(ctx->rowcarry.ensure(units * nj2 * 2 * ks));
-    CK(ctx->trace.ensure((size_t)n * tcap));
     CK(ctx->misc.ensure(3 + n));                      // err, nact, it, act[n]
     CK(ctx->counters.ensure(8 * kCounterSlots));
     CK(ctx->counts.ensure(4 * (size_t)n));
     const size_t dsz = ctx->geo_p.ds.size() + ctx->geo_u.ds.size() + ctx->geo_v.ds.size();
     CK(ctx->diag.ensure(dsz));
     CK(ctx->bcl.ensure(wptr.size() + wev.size() + sptr.size() + sev.size() + 4));
-    const bool has_veg = s->veg && s->veg_mask;
-    if (has_veg) CK(ctx->veg.ensure((size_t)ncols * ks));
 
     cudaStream_t st = ctx->stream;
     CK(cudaEventRecord(ctx->ev[0], st));
@@ -1038,10 +1096,10 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
         CK(ctx->dtab.ensure(dt.size()));
         ctx->dcb = DiagChainBufs{};
         if (const int lv = (ctx->chains & 2) ? diag_chain_levels(NKK) : 0) {
-            // DIV/DTIME for as many situations at a time as fit 4 GB; without memory for the planes the
+            // DIV/DTIME for as many situations at a time as fit kDiagBytes; without memory for the planes the
             // diagonal-claim wavefront below
             const size_t unit = (size_t)ncols * 64 * (lv / 2);
-            const int units = set_units(n, ((size_t)4 << 30) / (unit * sizeof(float)));
+            const int units = set_units(n, kDiagBytes / (unit * sizeof(float)));
             cudaError_t e = ctx->ddpm.ensure(unit * n);
             if (e == cudaSuccess) e = ctx->ddiv.ensure(unit * units);
             if (e == cudaSuccess) e = ctx->dwords.ensure(diag_chain_words(NII, NJJ, lv) * n);

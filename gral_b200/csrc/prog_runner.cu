@@ -7,14 +7,15 @@
 // wavefront kernels claim their tasks in dependency order from an atomic counter, so they need no
 // co-residency and make progress next to each other's launches.
 //
-// Admission and packing: the instances are ordered by their device footprint, largest first.
-// The largest is loaded and its footprint measured; the others' are scaled from it by their field
-// sizes, and K slots are opened for the largest K instances whose footprints fit the HBM budget
-// together.  Those K loads run one after the other before any solve starts, so every device
-// allocation happens while nothing else runs (an allocation can wait for work in flight on the
+// Admission and packing: the instances are ordered by the device bytes of their loads (load_size), largest
+// first.  As many slots are opened, K at most, as fit the HBM budget together, each with every buffer
+// as large as its first instance or any of the instances queued behind the first K needs it: one with more
+// columns but fewer levels has the smaller fields and the larger column records.  The slots' buffers and
+// first loads are made one after the other before any solve starts, so the device
+// allocations happen while nothing else runs (an allocation can wait for work in flight on the
 // device).  Then each slot's thread solves its instance and takes the next largest one left from a
-// shared queue as soon as it is done, loading it into the buffers of its first (larger) instance:
-// no slot waits for another, and the memory in use never exceeds what was admitted.
+// shared queue as soon as it is done, loading it into the slot's buffers: no slot waits for
+// another, and the memory in use stays within what was admitted.
 #include <algorithm>
 #include <atomic>
 #include <numeric>
@@ -51,15 +52,6 @@ void drop_if_failed(gral_ctx *&ctx, int rc) {
     ctx = nullptr;
 }
 
-// Device bytes of one instance's load, up to a common factor: the solver fields and row carry
-// ([col][KS] floats, ten fields), the staging copies ([col][NKK+2], three fields) and the
-// per-column tables.
-double footprint_units(const gral_params &q) {
-    const double ncols = (double)(q.nii + 2) * (q.njj + 2);
-    const double ks = (double)(((q.kadvmax + 2) + 7) / 8 * 8);
-    return ncols * (10.0 * ks + 3.0 * (q.nkk + 2) + 16.0);
-}
-
 }  // namespace
 
 extern "C" int gral_prog_solve_instances(int32_t n, const gral_params *p, const gral_static *s, gral_fields *f,
@@ -74,12 +66,7 @@ extern "C" int gral_prog_solve_instances(int32_t n, const gral_params *p, const 
         dims[3] = std::max(dims[3], p[b].kadvmax);
         status[b] = GRAL_EINVAL;
     }
-    std::vector<int> order(n);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int a, int b) { return footprint_units(p[a]) > footprint_units(p[b]); });
-
-    size_t free0 = 0, total = 0, free1 = 0;
+    size_t free0 = 0, total = 0;
     if (cudaMemGetInfo(&free0, &total) != cudaSuccess) {
         cudaGetLastError();
         return GRAL_ENODEV;
@@ -89,29 +76,49 @@ extern "C" int gral_prog_solve_instances(int32_t n, const gral_params *p, const 
     std::vector<gral_ctx *> slot(1, nullptr);
     int rc = gral_prog_create(dims[0], dims[1], dims[2], dims[3], 1, &slot[0]);
     if (rc != GRAL_OK) return rc;
-    // the largest instance is loaded first; its measured footprint scales the others'
-    const int first_rc = gral_prog_load(slot[0], 1, p + order[0], s + order[0], f + order[0]);
-    cudaMemGetInfo(&free1, &total);
-    const double bytes0 = (double)std::max<size_t>(free0 > free1 ? free0 - free1 : 0, 64u << 20) * 1.1;
-    const double per_unit = bytes0 / footprint_units(p[order[0]]);
-    const double budget = hbm_bytes ? (double)hbm_bytes : 0.9 * (double)free0;
-    int K = 1;
-    double used = bytes0;
-    while (K < std::min(n, max_concurrent)) {
-        const double next = per_unit * footprint_units(p[order[K]]);
-        if (used + next > budget) break;
-        used += next;
-        ++K;
+
+    std::vector<LoadSize> size(n);
+    std::vector<size_t> bytes(n);
+    for (int b = 0; b < n; ++b) {
+        // an instance that its load will refuse needs nothing
+        if (p[b].nii < 4 || p[b].njj < 4 || p[b].nkk < 3 || p[b].kadvmax < 2 || p[b].iteration_steps_max < 1) continue;
+        size[b] = load_size(slot[0], 1, p[b], s[b].veg && s[b].veg_mask);
+        bytes[b] = load_bytes(slot[0], size[b]);
     }
+    std::vector<int> order(n);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return bytes[a] > bytes[b]; });
+    // later[q]: the largest of each buffer over the instances from position q on
+    std::vector<LoadSize> later(n + 1);
+    for (int q = n - 1; q >= 0; --q) {
+        later[q] = later[q + 1];
+        later[q].cover(size[order[q]]);
+    }
+    const size_t budget = hbm_bytes ? (size_t)hbm_bytes : free0 / 10 * 9;
+    // the buffers of slot t of K: its first instance's, and those of every instance that may follow
+    auto slot_size = [&](int t, int K) {
+        LoadSize z = size[order[t]];
+        z.cover(later[K]);
+        return z;
+    };
+    auto fits = [&](int K) {
+        size_t sum = 0;
+        for (int t = 0; t < K && sum <= budget; ++t) sum += load_bytes(slot[0], slot_size(t, K));
+        return sum <= budget;
+    };
+    int K = std::min(n, max_concurrent);
+    while (K > 1 && !fits(K)) --K;
     slot.resize(K, nullptr);
 
-    // the first K loads, one after the other, before any solve
+    // the slots' buffers and first loads, one after the other, before any solve
     std::vector<int> rcs(K, GRAL_OK);
-    rcs[0] = first_rc;
-    for (int t = 1; t < K; ++t) {
+    for (int t = 0; t < K; ++t) {
         const int b = order[t];
-        rcs[t] = gral_prog_create(dims[0], dims[1], dims[2], dims[3], 1, &slot[t]);
-        if (rcs[t] == GRAL_OK) rcs[t] = gral_prog_load(slot[t], 1, p + b, s + b, f + b);
+        if (t > 0) rcs[t] = gral_prog_create(dims[0], dims[1], dims[2], dims[3], 1, &slot[t]);
+        if (rcs[t] != GRAL_OK) continue;
+        reserve_load(slot[t], slot_size(t, K));     // without the memory the load takes what it needs itself
+        cudaGetLastError();
+        rcs[t] = gral_prog_load(slot[t], 1, p + b, s + b, f + b);
     }
     // each slot solves its instance, then takes the next largest one left
     std::atomic<int> next{K};

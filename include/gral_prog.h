@@ -166,9 +166,11 @@ int gral_prog_solve_batch_devices(int32_t ndev, const int32_t *devices, int32_t 
  * device footprint, largest first; K slots (each a context, stream and host thread) take the K
  * largest, whose loads run one after the other, then every slot solves its instance and takes the
  * next largest one left as soon as it is done, reusing its buffers.  K is max_concurrent, further
- * limited to the largest instances whose footprints fit in hbm_bytes of device memory together
- * (0: 90 % of the free memory at the call; the largest instance is loaded first and its measured
- * footprint scales the others' by their field sizes).  status[b] receives
+ * limited so that the slots' buffers, each as large as any instance the slot may take needs it, fit
+ * in hbm_bytes of device memory together (0: 90 % of the free memory at the call; at least one slot
+ * is opened).  On row chains a single instance of a few hundred columns a side already keeps a GPU
+ * busy, and solving them side by side need not be faster than one call after the other; it pays for small
+ * grids.  status[b] receives
  * instance b's return code (the error text of a failed instance is not kept); the call returns
  * GRAL_OK when every instance succeeded, else the code of the first failed instance in index
  * order.  stats may be NULL. */
