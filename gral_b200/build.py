@@ -16,7 +16,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgralprog.so")
 SOURCES = ["prog_host.cu", "prog_pages.cu", "prog_gs.cu", "prog_chain.cu", "prog_chain_scalar.cu", "prog_chain_diag.cu", "prog_kernels.cu", "prog_gff.cu", "prog_prep.cu", "prog_wind.cu", "prog_runner.cu", "prog_noalloc.cu", "prog_adjoint.cu"]
-HEADERS = ["prog_common.cuh", "prog_ctx.cuh", "unit_sets.h", "prog_pages.cuh", "prog_chain.cuh", "prog_kernels.cuh", "prog_level.cuh", "prog_quot.cuh", "prog_gff.cuh", "prog_prep.cuh", "adj_level.cuh", "adj_chain.cuh"]
+HEADERS = ["prog_common.cuh", "prog_ctx.cuh", "batch_rules.h", "prog_pages.cuh", "prog_chain.cuh", "prog_kernels.cuh", "prog_level.cuh", "prog_quot.cuh", "prog_gff.cuh", "prog_prep.cuh", "adj_level.cuh", "adj_chain.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

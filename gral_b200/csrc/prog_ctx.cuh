@@ -11,7 +11,7 @@
 #include "gral_prog.h"
 #include "prog_common.cuh"
 #include "prog_kernels.cuh"
-#include "unit_sets.h"
+#include "batch_rules.h"
 
 namespace gral {
 

@@ -177,20 +177,9 @@ Geom make_geom(int ia, int ni, int ja, int nj) {
     return G;
 }
 
-// Whether a batch runs faster in the interleaved layout.  A batched sweep waits for its wavefront (a per
-// diagonal) and works through its groups of 32 (b per column and group); the row chains take p per
-// column and situation.  ms of an iteration, fitted to 100x100 .. 400x400 grids with 32 to 144
-// situations; measured row chains / interleaved, model 1: 48 of 100x100 3.9 / 8.4, 64 of 200x200 20.7 /
-// 20.3; model 2: 64 of 100x100 11.0 / 14.2, of 200x200 42.8 / 38.9; model 0: 6.9 / 8.6 and 25.7 / 22.9.
-bool interleaved_pays(int n, int nii, int njj, int model) {
-    if (n < 32) return false;
-    static const double P[3] = {9.9e-6, 7.9e-6, 16.4e-6}, A[3] = {0.042, 0.033, 0.072}, B[3] = {0.049e-3, 0.094e-3, 0.074e-3};
-    const double cols = (double)nii * njj, groups = (n + 31) / 32;
-    return P[model] * n * cols > A[model] * (nii + njj) + B[model] * groups * cols;
-}
-
 bool interleaved(const gral_ctx *ctx, int n, const gral_params &p) {
-    return ctx->il_min_batch > 0 ? n >= ctx->il_min_batch : interleaved_pays(n, p.nii, p.njj, p.turbulence_model);
+    if (ctx->il_min_batch > 0) return n >= ctx->il_min_batch;
+    return interleaved_pays(n, p.nii, p.njj, std::min(p.vert_cells_ff, p.nkk - 1), p.turbulence_model);
 }
 
 int validate(gral_ctx *ctx, int n, const gral_params *p, const gral_static *s, const gral_fields *f) {

@@ -3,7 +3,7 @@
 // smallest set.  Prints "ok" or the first failure.
 #include <cstdio>
 
-#include "unit_sets.h"
+#include "batch_rules.h"
 
 using namespace gral;
 
