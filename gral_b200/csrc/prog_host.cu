@@ -177,6 +177,26 @@ Geom make_geom(int ia, int ni, int ja, int nj) {
     return G;
 }
 
+// the buffers that only the row chains need (the iteration epoch stays, so that later words are new)
+void release_chains(gral_ctx *ctx) {
+    ctx->crec.release(); ctx->cwords.release(); ctx->cptab.release();
+    ctx->ddpm.release(); ctx->ddiv.release(); ctx->dwords.release();
+    ctx->adj_rec.release(); ctx->adj_plane.release(); ctx->adj_word.release();
+}
+
+// a buffer that a load cannot do without: where there is no memory for it, what an earlier load took for the
+// chains is given back first
+template <class T>
+cudaError_t ensure_first(gral_ctx *ctx, DevBuf<T> &buf, size_t count) {
+    cudaError_t e = buf.ensure(count);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        release_chains(ctx);
+        e = buf.ensure(count);
+    }
+    return e;
+}
+
 bool interleaved(const gral_ctx *ctx, int n, const gral_params &p) {
     if (ctx->il_min_batch > 0) return n >= ctx->il_min_batch;
     return interleaved_pays(n, p.nii, p.njj, std::min(p.vert_cells_ff, p.nkk - 1), p.turbulence_model);
@@ -598,10 +618,10 @@ int run_diagnostic(gral_ctx *ctx) {
     return GRAL_OK;
 }
 
-// Buffers of the row-chain schedule: records for as many situations at a time as fit kChainBytes (the
-// situations are independent, so sets of them run one after the other), the words between strips and
-// the elimination table of the pressure sweep, built here.  If they do not fit on the device the
-// strip schedule, which needs none of them, stays the default.
+// Buffers of the row-chain schedule: records for as many situations at a time as fit kChainBytes and a
+// quarter of the free memory (the situations are independent, so sets of them run one after the
+// other), the words between strips and the elimination table of the pressure sweep, built here.  If
+// they do not fit on the device the strip schedule, which needs none of them, stays the default.
 int reserve_chain(gral_ctx *ctx) {
     ctx->chain_ok = false;
     ctx->ka.epoch = nullptr;
@@ -609,7 +629,11 @@ int reserve_chain(gral_ctx *ctx) {
     cudaStream_t st = ctx->stream;
     const size_t unit = chain_record_bytes(ctx->model) * ctx->ncols;
     const size_t words = chain_unit_words(ctx->nii, ctx->njj);
-    size_t fit = kChainBytes / unit;
+    // records grow to a quarter of the free memory at most: other contexts and this one's later calls need theirs
+    size_t most = kChainBytes, held = ctx->crec.n * sizeof(float2), free0 = 0, total = 0;
+    if (unit * set_units(ctx->nb, most / unit) > held && cudaMemGetInfo(&free0, &total) == cudaSuccess)
+        most = std::min(most, std::max(held, (free0 + held) / 4));
+    size_t fit = most / unit;
     if (const char *v = std::getenv("GRAL_PROG_CHAIN_UNITS")) fit = std::min(fit, (size_t)std::max(1, std::atoi(v)));
     int units = set_units(ctx->nb, fit);
     const size_t had = ctx->cwords.n;
@@ -773,7 +797,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
     // of the reference column that the scalars below need come back to the host.
     if (ctx->flat_met) {
         const size_t ssz0 = (size_t)ncols * nk2;
-        CK(ctx->stage.ensure(ssz0 * ((ctx->model != 1) ? 5 : 3) * n));
+        CK(ensure_first(ctx, ctx->stage, ssz0 * ((ctx->model != 1) ? 5 : 3) * n));
         cudaStream_t st0 = ctx->stream;
         PrepBufs &pb = ctx->prep;
         CK(pb.cutk.ensure(ncols));
@@ -922,7 +946,7 @@ int gral_prog_load(gral_ctx *ctx, int32_t n, const gral_params *p, const gral_st
     const LoadSize z = load_size(ctx, n, p0, has_veg);
     cudaError_t ze = cudaSuccess;
     load_buffers(*ctx, [&](int q, auto &buf) {
-        if (q < LB_BASE && ze == cudaSuccess) ze = buf.ensure(z.n[q]);
+        if (q < LB_BASE && ze == cudaSuccess) ze = ensure_first(ctx, buf, z.n[q]);
     });
     CK(ze);
     CK(ctx->tables.ensure(7 * ks));
