@@ -1463,6 +1463,9 @@ int gral_prog_vjp_forward(gral_ctx *ctx, const gral_params *p, const gral_static
                                     st));
     } else {
         const int nck = (iterations + checkpoint_every - 1) / checkpoint_every;
+        CK(ctx->adj_ckpt.ensure((size_t)nck * NCKPT * fsz));
+        CK(ctx->adj_cksit.ensure(nck));
+        CK(ctx->adj_ckit.ensure(nck));
         // the last segment is reversed first: its states are kept while it runs, where there is room, and
         // gral_prog_vjp has nothing to recompute before it starts
         const size_t buf = keep_buffers(nck) * checkpoint_every, nevk = (size_t)std::max(nev[0] + nev[1], 1) * a.ks;
@@ -1473,9 +1476,6 @@ int gral_prog_vjp_forward(gral_ctx *ctx, const gral_params *p, const gral_static
         const bool keep = e == cudaSuccess;
         const size_t slot0 = (size_t)((nck - 1) % keep_buffers(nck)) * checkpoint_every;
         if (keep) CK(cudaMemsetAsync(ctx->adj_bits.p, 0, buf * nevk, st));
-        CK(ctx->adj_ckpt.ensure((size_t)nck * NCKPT * fsz));
-        CK(ctx->adj_cksit.ensure(nck));
-        CK(ctx->adj_ckit.ensure(nck));
         CK(cudaEventRecord(ctx->ev[0], st));
         for (int it = 0; it < iterations; ++it) {
             if (it % checkpoint_every == 0) CK_RC(save_checkpoint(ctx, it / checkpoint_every));
