@@ -241,8 +241,9 @@ int validate(gral_ctx *ctx, int n, const gral_params *p, const gral_static *s, c
     return GRAL_OK;
 }
 
-// bounds of the column records that the row chains hold at once and of the diagnostic step's DIV/DTIME
-constexpr size_t kChainBytes = (size_t)16 << 30, kDiagBytes = (size_t)4 << 30;
+// bounds of the column records that the row chains hold at once (the second whatever memory is free) and of the
+// diagnostic step's DIV/DTIME
+constexpr size_t kChainBytes = (size_t)16 << 30, kChainBytesSmall = (size_t)512 << 20, kDiagBytes = (size_t)4 << 30;
 
 // the plain mode of the row-chain schedule, after the fused strips
 int kChainMode() { return 2 + strip_num_variants(); }
@@ -629,10 +630,11 @@ int reserve_chain(gral_ctx *ctx) {
     cudaStream_t st = ctx->stream;
     const size_t unit = chain_record_bytes(ctx->model) * ctx->ncols;
     const size_t words = chain_unit_words(ctx->nii, ctx->njj);
-    // records grow to a quarter of the free memory at most: other contexts and this one's later calls need theirs
+    // records beyond half a gigabyte grow to a quarter of the free memory at most: other contexts and this
+    // one's later calls need theirs
     size_t most = kChainBytes, held = ctx->crec.n * sizeof(float2), free0 = 0, total = 0;
-    if (unit * set_units(ctx->nb, most / unit) > held && cudaMemGetInfo(&free0, &total) == cudaSuccess)
-        most = std::min(most, std::max(held, (free0 + held) / 4));
+    if (unit * set_units(ctx->nb, most / unit) > std::max(held, kChainBytesSmall) && cudaMemGetInfo(&free0, &total) == cudaSuccess)
+        most = std::min(most, std::max({held, kChainBytesSmall, (free0 + held) / 4}));
     size_t fit = most / unit;
     if (const char *v = std::getenv("GRAL_PROG_CHAIN_UNITS")) fit = std::min(fit, (size_t)std::max(1, std::atoi(v)));
     int units = set_units(ctx->nb, fit);
