@@ -478,7 +478,8 @@ struct PressChain {
         const float2 *t = b.ptab + ((size_t)(IS == 1 ? 0 : 1) * a.ncols + col) * a.ks;
         div = reinterpret_cast<const float2 *>(d) + l;
         tab = reinterpret_cast<const float4 *>(t) + l;
-        // lines of 128 bytes of the two runs (they need not start on one): lanes 0-3 and 4-9
+        // lines of 128 bytes of the two runs, lanes 0-3 and 4-7 (a run that does not start on a line leaves the
+        // last bit of it to the load)
         line = lane < 4 ? reinterpret_cast<const char *>(d) + 128 * lane : reinterpret_cast<const char *>(t) + 128 * (lane - 4);
         on0 = lane < 4 ? 128 * lane < a.ks * 4 : (lane < 8 && 128 * (lane - 4) < a.ks * 8);
         step_line = (long long)JS * M * a.ks * (lane < 4 ? 4 : 8);

@@ -275,7 +275,8 @@ class PrognosticSolver:
 
     def flat_init(self, grid: dict, cutk: np.ndarray, dzk: np.ndarray, hokart: np.ndarray, met: MetProfile,
                   advdom: Optional[np.ndarray] = None):
-        """Flat-terrain set-up of one situation; returns (kkart, ahk, kadvmax, FieldArrays)."""
+        """Flat-terrain set-up of one situation; returns (kkart, ahk, kadvmax, FieldArrays).  The three fields are
+        views of one block: copy a field to keep it without the others."""
         nii, njj, nkk = grid["nii"], grid["njj"], grid["nkk"]
         g = GralFlatGrid(**grid)
         cutk, dzk, hokart = (np.ascontiguousarray(a, np.float32) for a in (cutk, dzk, hokart))
@@ -313,7 +314,8 @@ class PrognosticSolver:
     def wind_at(self, situation: int, grid: dict, dzk: Optional[np.ndarray], hokart: Optional[np.ndarray],
                 particles: np.ndarray, met: Optional[MetProfile] = None):
         """U, V, W and IndexK at particle positions (``PARTICLE_DTYPE`` records), interpolated from
-        the stored fields of `situation` as Zeitschleife.IntWindCalculate does."""
+        the stored fields of `situation` as Zeitschleife.IntWindCalculate does.  The four results are views
+        of one block: copy one to keep it without the others."""
         p = np.ascontiguousarray(particles, dtype=PARTICLE_DTYPE)
         n = p.size
         out = np.empty((4, n), np.float32)     # one block, as in flat_init
