@@ -168,9 +168,9 @@ int gral_prog_solve_batch_devices(int32_t ndev, const int32_t *devices, int32_t 
  * next largest one left as soon as it is done, reusing its buffers.  K is max_concurrent, further
  * limited so that the slots' buffers, each as large as any instance the slot may take needs it, fit
  * in hbm_bytes of device memory together (0: 90 % of the free memory at the call; at least one slot
- * is opened).  A few slots are worth more than many: 16 grids of 24 to 200 columns a side took 0.5 to
- * 0.7 of one slot's time in four slots and 0.5 to 1.1 in 16; a larger grid on row chains already keeps
- * the GPU busy by itself.  status[b] receives
+ * is opened).  A few slots give most of the gain: 16 grids of 24 to 200 columns a side took 0.5 to 0.7
+ * of one slot's time in four slots and 0.5 to 1.1 in 16, 16 grids of 131 to 467 columns 0.7 and 0.6.
+ * status[b] receives
  * instance b's return code (the error text of a failed instance is not kept); the call returns
  * GRAL_OK when every instance succeeded, else the code of the first failed instance in index
  * order.  stats may be NULL. */
